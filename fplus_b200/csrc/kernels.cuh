@@ -1230,220 +1230,6 @@ __global__ void __launch_bounds__(640) k_front_lu2(const T *__restrict__ W, int6
     front_lu2_body<T>(W, ld, nrows, npiv, nri, fcol, colmax, pivot_rel, rowid, Lout, perm, p_lu, st, front, pa);
 }
 
-// Blocked partial-pivot LU of a front's pivot block (nrows <= 128, npiv <= 64; one CTA of 256 threads): 8-column panels
-// pivoted by warps 0-3 (thread i < 128 holds row i's eight panel entries in registers; per pivot step every warp posts its
-// candidate with the candidate row's panel entries, one 128-thread barrier, and every thread makes the same decision),
-// then the panel's pivot rows' U for the later columns by an 8-step forward substitution (a thread per column), then
-// the rank-8 update of every later column as FP64 tensor-core products (mma m8n8k4) of the masked multipliers (rows
-// already pivoted read zero) and the pivot rows' U.  Rows never move: a row pivoted at step j is tagged j, and the block
-// goes out in the final order at the end.  The pivots are those of the step-by-step elimination (the update of a later
-// column sums the panel's eight products in another order, so the values agree to rounding).
-constexpr int LU5_THREADS = 256, LU5_PB = 8, LU5_LMLD = 132;
-
-template <typename T> struct Lu5Cand {
-    unsigned long long key;
-    long long rid;
-    int row, pad;
-    T val, inv;
-    T u[LU5_PB];
-};
-
-// dynamic shared memory: the block, row ids, thresholds and their keys, the masked multipliers (two planes for complex),
-// the final order
-static inline size_t front_lu5_smem(int64_t nrows, int64_t npiv, int64_t vs)
-{
-    return (size_t)(nrows * npiv * vs + nrows * 8 + npiv * 16 + (vs / 8) * LU5_PB * LU5_LMLD * 8 + nrows * 4);
-}
-
-template <typename T>
-__device__ __forceinline__ void front_lu5_body(const T *__restrict__ W, int64_t ld, int nrows, int npiv, int nri,
-                                               int64_t fcol, const double *__restrict__ colmax, double pivot_rel,
-                                               int64_t *__restrict__ rowid, T *__restrict__ Lout, int *__restrict__ perm,
-                                               int64_t *__restrict__ p_lu, DevStatus *st, int64_t front, const PivotAsm &pa)
-{
-    constexpr bool CP = VT<T>::cplx_;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *A = reinterpret_cast<T *>(smem_raw);                        // npiv x nrows, column-major: A[c * nrows + i]
-    int64_t *rid = reinterpret_cast<int64_t *>(A + (size_t)npiv * nrows);
-    double *thr = reinterpret_cast<double *>(rid + nrows);
-    unsigned long long *thk = reinterpret_cast<unsigned long long *>(thr + npiv);
-    double *Lmr = reinterpret_cast<double *>(thk + npiv);         // masked multipliers: Lm[k][row] at k * LU5_LMLD + row
-    double *Lmi = Lmr + (CP ? LU5_PB * LU5_LMLD : 0);
-    int *sperm = reinterpret_cast<int *>(Lmr + (CP ? 2 : 1) * LU5_PB * LU5_LMLD);
-    __shared__ Lu5Cand<T> cand[2][4];
-    __shared__ int prow[LU5_PB], s_stop, wcnt[4];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_stop = st->code != 0;
-    stage_pivot_block<T>(A, rid, W, ld, nrows, npiv, rowid, pa, tid, LU5_THREADS);
-    for (int c = tid; c < npiv; c += LU5_THREADS) {
-        thr[c] = pivot_rel * colmax[fcol + c];
-        thk[c] = pivkey_of_modulus<T>(2.0 * thr[c]);
-    }
-    __syncthreads();
-    if (s_stop) return;
-    const bool pg = tid < 128;                                     // the panel group: thread i holds row i
-    const int i = tid;
-    const long long myrid = pg && i < nrows ? (long long)rid[i] : LLONG_MAX;
-    bool live = pg && i < nrows;
-    int mytag = INT_MAX;
-    for (int c0 = 0; c0 < npiv; c0 += LU5_PB) {
-        const int w = npiv - c0 < LU5_PB ? npiv - c0 : LU5_PB;   // pivot steps of this panel
-        if (pg) {
-            T pv[LU5_PB];
-#pragma unroll
-            for (int s = 0; s < LU5_PB; s++) pv[s] = i < nrows && s < w ? A[(c0 + s) * nrows + i] : VT<T>::zero();
-#pragma unroll
-            for (int s = 0; s < LU5_PB; s++) {
-                if (s >= w) break;
-                const int par = s & 1, j = c0 + s;
-                // this warp's candidate for column j, posted with its row's panel entries
-                const unsigned long long key = live ? pivkey(pv[s]) : 0ull;
-                const T xinv = key != 0ull ? recip(pv[s]) : VT<T>::zero();
-                const unsigned long long mk = warp_max_key(key);
-                unsigned cnd = __ballot_sync(0xffffffffu, key != 0ull && key == mk);
-                if (cnd != 0u && (cnd & (cnd - 1u)) != 0u) {
-                    long long r2 = (cnd >> lane) & 1u ? myrid : LLONG_MAX;
-                    for (int o = 16; o > 0; o >>= 1) { const long long t = __shfl_xor_sync(0xffffffffu, r2, o); r2 = t < r2 ? t : r2; }
-                    cnd = __ballot_sync(0xffffffffu, ((cnd >> lane) & 1u) && myrid == r2);
-                }
-                const int wl = cnd != 0u ? __ffs(cnd) - 1 : 0;
-                if (lane == wl) {
-                    Lu5Cand<T> &cd = cand[par][warp];
-                    cd.key = cnd != 0u ? mk : 0ull; cd.rid = cnd != 0u ? myrid : LLONG_MAX; cd.row = cnd != 0u ? i : -1;
-                    cd.val = pv[s]; cd.inv = xinv;
-#pragma unroll
-                    for (int q = 0; q < LU5_PB; q++) cd.u[q] = pv[q];
-                }
-                named_bar(1, 128);
-                // the winner (every thread of the group the same): the largest key, ties to the smaller row of B
-                int bs = 0;
-                unsigned long long bk = cand[par][0].key;
-                long long br = cand[par][0].rid;
-#pragma unroll
-                for (int q = 1; q < 4; q++) {
-                    const unsigned long long k = cand[par][q].key;
-                    const long long r = cand[par][q].rid;
-                    if (k > bk || (k == bk && r < br)) { bk = k; br = r; bs = q; }
-                }
-                const int bi = cand[par][bs].row;
-                const T pvw = cand[par][bs].val, inv = cand[par][bs].inv;
-                int stop = 0;
-                if (bi < 0 || bk == 0ull || (bk < thk[j] && vabs(pvw) < thr[j])) stop = 1;
-                else if (bi >= nri) stop = 2;
-                if (stop) {
-                    if (tid == 0) {
-                        if (stop == 1) set_status(st, ST_SINGULAR, fcol + j, bi >= 0 ? vabs(pvw) : 0.0, thr[j]);
-                        else set_status(st, ST_BORDER, front, vabs(pvw), thr[j]);
-                        s_stop = 1;
-                    }
-                    break;                                         // (every thread of the group the same)
-                }
-                if (i == bi) { mytag = j; live = false; prow[s] = i; }
-                if (live) {
-                    const T l = mul(pv[s], inv);
-                    pv[s] = l;
-#pragma unroll
-                    for (int q = s + 1; q < LU5_PB; q++) pv[q] = sub(pv[q], mul(l, cand[par][bs].u[q]));
-                }
-            }
-            // the panel back into the block; the masked multipliers (zero for every row pivoted so far)
-#pragma unroll
-            for (int s = 0; s < LU5_PB; s++) {
-                if (i < nrows && s < w) A[(c0 + s) * nrows + i] = pv[s];
-                const T lm = live && s < w ? pv[s] : VT<T>::zero();
-                if constexpr (CP) { Lmr[s * LU5_LMLD + i] = lm.x; Lmi[s * LU5_LMLD + i] = lm.y; } else Lmr[s * LU5_LMLD + i] = lm;
-            }
-        }
-        __syncthreads();
-        if (s_stop) return;
-        const int t0 = c0 + w, T_ = npiv - t0;                     // the later columns
-        if (T_ <= 0) continue;
-        // the pivot rows' U for the later columns: forward substitution with the panel's unit-lower L (a thread per column)
-        for (int c = t0 + tid; c < npiv; c += LU5_THREADS) {
-            T u[LU5_PB];
-#pragma unroll
-            for (int k = 0; k < LU5_PB; k++) u[k] = k < w ? A[c * nrows + prow[k]] : VT<T>::zero();
-#pragma unroll
-            for (int k = 1; k < LU5_PB; k++) {
-                if (k >= w) break;
-                T acc = u[k];
-#pragma unroll
-                for (int q = 0; q < k; q++) acc = sub(acc, mul(A[(c0 + q) * nrows + prow[k]], u[q]));
-                u[k] = acc;
-                A[c * nrows + prow[k]] = acc;
-            }
-        }
-        __syncthreads();
-        // the rank-w update of every later column on the FP64 tensor cores: A[r, c] -= sum_k Lm[k][r] U[k, c]
-        // (item = an 8-row x 8-column fragment; rows already pivoted have zero multipliers and stay as they are)
-        {
-            const int rf = (nrows + 7) >> 3, cf = (T_ + 7) >> 3;
-            for (int p = warp; p < rf * cf; p += LU5_THREADS / 32) {
-                const int r0 = 8 * (p % rf), cb = t0 + 8 * (p / rf);
-                double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-                const int am = r0 + (lane >> 2), bn = cb + (lane >> 2);
-#pragma unroll
-                for (int ks = 0; ks < LU5_PB; ks += 4) {
-                    const int k = ks + (lane & 3);
-                    const bool kin = k < w;
-                    const double ar = kin && am < nrows ? Lmr[k * LU5_LMLD + am] : 0.0;
-                    const double ai = CP && kin && am < nrows ? Lmi[k * LU5_LMLD + am] : 0.0;
-                    T bv = kin && bn < npiv ? A[bn * nrows + prow[k < w ? k : 0]] : VT<T>::zero();
-                    double brr, bii;
-                    if constexpr (CP) { brr = bv.x; bii = bv.y; } else { brr = bv; bii = 0.0; }
-                    dmma(a0, a1, ar, brr);
-                    if constexpr (CP) {
-                        dmma(b0, b1, ar, bii);
-                        dmma(a0, a1, ai, -bii);
-                        dmma(b0, b1, ai, brr);
-                    }
-                }
-                const int cr = r0 + (lane >> 2), cc = cb + 2 * (lane & 3);
-                if (cr < nrows) {
-                    if (cc < npiv) {
-                        T *x = A + cc * nrows + cr;
-                        if constexpr (CP) *x = cplx{x->x - a0, x->y - b0}; else *x = *x - a0;
-                    }
-                    if (cc + 1 < npiv) {
-                        T *x = A + (cc + 1) * nrows + cr;
-                        if constexpr (CP) *x = cplx{x->x - a1, x->y - b1}; else *x = *x - a1;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // the final order: pivot rows at their step, the others after them in block order (warps 0-3, a row each)
-    if (pg) {
-        const bool un = i < nrows && mytag == INT_MAX;
-        const unsigned bal = __ballot_sync(0xffffffffu, un);
-        if (lane == 0) wcnt[warp] = __popc(bal);
-        named_bar(1, 128);
-        int k0 = npiv;
-        for (int q = 0; q < warp; q++) k0 += wcnt[q];
-        const int k = un ? k0 + __popc(bal & ((1u << lane) - 1u)) : mytag;
-        if (i < nrows) {
-            sperm[k] = i;
-            perm[k] = i;
-            rowid[k] = myrid;
-            if (k < npiv) p_lu[fcol + k] = myrid;
-        }
-    }
-    __syncthreads();
-    const int ne = npiv * nrows;
-    for (int e = tid; e < ne; e += LU5_THREADS) { const int kk = e % nrows, c = e / nrows; Lout[e] = A[c * nrows + sperm[kk]]; }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(LU5_THREADS) k_front_lu5(const T *__restrict__ W, int64_t ld, int nrows, int npiv, int nri,
-                                                            int64_t fcol, const double *__restrict__ colmax, double pivot_rel,
-                                                            int64_t *__restrict__ rowid, T *__restrict__ Lout,
-                                                            int *__restrict__ perm, int64_t *__restrict__ p_lu, DevStatus *st,
-                                                            int64_t front, PivotAsm pa)
-{
-    front_lu5_body<T>(W, ld, nrows, npiv, nri, fcol, colmax, pivot_rel, rowid, Lout, perm, p_lu, st, front, pa);
-}
-
 // Blocked partial-pivot LU of a front's pivot block in shared memory (nrows <= 128, npiv <= 64; one CTA of LU3_THREADS):
 // the same elimination as k_front_lu2 in panels of LU3_PB columns with a one-panel look-ahead.
 //   warp 0 (the panel warp)  factors panel p = columns [c0, c1) with its rows in registers (row i in lane i % 32, slot
@@ -3916,21 +3702,6 @@ __global__ void __launch_bounds__(640) k_bat_lu2(const FcFront *__restrict__ fc,
     PivotAsm pa;
     pa.on = 0;
     front_lu2_body<T>(Wbase + F.wofs, F.nr, (int)F.nr, (int)F.np, (int)F.nri, F.f, colmax, pivot_rel, rowid_all + F.row_off,
-                      La + F.L_off, permall + F.row_off, p_lu, st, fi, pa);
-}
-
-// the same with the blocked pivot-block LU (the body of k_front_lu5)
-template <typename T>
-__global__ void __launch_bounds__(LU5_THREADS) k_bat_lu5(const FcFront *__restrict__ fc, const int *__restrict__ list,
-                                                          const T *__restrict__ Wbase, const double *__restrict__ colmax,
-                                                          double pivot_rel, int64_t *__restrict__ rowid_all, T *__restrict__ La,
-                                                          int *__restrict__ permall, int64_t *__restrict__ p_lu, DevStatus *st)
-{
-    const int fi = list[blockIdx.x];
-    const FcFront F = fc[fi];
-    PivotAsm pa;
-    pa.on = 0;
-    front_lu5_body<T>(Wbase + F.wofs, F.nr, (int)F.nr, (int)F.np, (int)F.nri, F.f, colmax, pivot_rel, rowid_all + F.row_off,
                       La + F.L_off, permall + F.row_off, p_lu, st, fi, pa);
 }
 

@@ -2,6 +2,7 @@
 // state of one factorization, and the launch sequences.
 #include "numeric.hpp"
 #include "kernels.cuh"
+#include "front_lu.cuh"
 #include "schur_tc.hpp"
 #include <algorithm>
 #include <cstring>
@@ -556,11 +557,13 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
     if ((rc = ensure_async(N, (void **)&N.rowid, &N.cap_rowid, (size_t)P.rows_total * 8, err, errlen))) return rc;
     if ((rc = ensure_async(N, (void **)&N.ipiv, &N.cap_ipiv, (size_t)(N.n > 0 ? N.n : 1) * 4, err, errlen))) return rc;
     if ((rc = ensure_async(N, (void **)&N.permall, &N.cap_permall, (size_t)(P.rows_total > 0 ? P.rows_total : 1) * 4, err, errlen))) return rc;
+    constexpr int LU6_TW = lu6_tallw(VT<T>::cplx_);
     static thread_local int attr_set = 0;
     if (!attr_set) {
         CK(cudaFuncSetAttribute(k_front_lu2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-        CK(cudaFuncSetAttribute(k_front_lu5<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_lu5_smem(128, 64, sizeof(T))));
-        CK(cudaFuncSetAttribute(k_bat_lu5<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_lu5_smem(128, 64, sizeof(T))));
+        CK(cudaFuncSetAttribute(k_front_lu6<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lu6_smem_max<T, 4>()));
+        CK(cudaFuncSetAttribute(k_front_lu6<T, LU6_TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, lu6_smem_max<T, LU6_TW>()));
+        CK(cudaFuncSetAttribute(k_bat_lu6<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lu6_smem_max<T, 4>()));
         CK(cudaFuncSetAttribute(k_front_lu3<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         CK(cudaFuncSetAttribute(k_trsm_warp<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         CK(cudaFuncSetAttribute(k_trsm_warp<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
@@ -755,15 +758,19 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             } else
                 k_front_lu3<T><<<1, LU3_THREADS, sm3, st>>>(W, ld, (int)nr, (int)np, (int)F.nri, F.f, N.colmax, pivot_rel,
                                                             N.rowid + F.row_off, Lf, perm, N.p_lu, N.st, fi, pa), note_launch();
-        } else if ((N.lu_variant & 3) == 1 && nr <= 128 && np <= 64) {
-            const size_t sm5 = front_lu5_smem(nr, np, vs);
+        } else if ((N.lu_variant & 3) == 2 && front_lu6_fits<T>(nr, np)) {
+            // the panel LU wherever shared memory holds its block: measured 2.0x (120 x 64 complex), 1.7x (120 x 64 real) and
+            // 2.5x (213 x 64 real) as fast as k_front_lu2, and never slower (3 x 2: 4.6 against 6.4 us)
+            auto lu6 = nr <= 128 ? k_front_lu6<T, 4> : k_front_lu6<T, LU6_TW>;
+            const int nt6 = front_lu6_threads(nr, np);
+            const size_t sm6 = front_lu6_smem(nr, np, vs);
             if (pa.on) {      // right after the child's tail head on the critical stream: overlap the launch
-                CK(launch_pdl(k_front_lu5<T>, 1, LU5_THREADS, sm5, st, (const T *)W, ld, (int)nr, (int)np, (int)F.nri, F.f,
+                CK(launch_pdl(lu6, 1, nt6, sm6, st, (const T *)W, ld, (int)nr, (int)np, (int)F.nri, F.f,
                               (const double *)N.colmax, pivot_rel, N.rowid + F.row_off, Lf, perm, N.p_lu, N.st, fi, pa));
                 note_launch();
             } else
-                k_front_lu5<T><<<1, LU5_THREADS, sm5, st>>>(W, ld, (int)nr, (int)np, (int)F.nri, F.f, N.colmax, pivot_rel,
-                                                            N.rowid + F.row_off, Lf, perm, N.p_lu, N.st, fi, pa), note_launch();
+                lu6<<<1, nt6, sm6, st>>>(W, ld, (int)nr, (int)np, (int)F.nri, F.f, N.colmax, pivot_rel, N.rowid + F.row_off, Lf, perm,
+                                         N.p_lu, N.st, fi, pa), note_launch();
         } else if (sm <= SMEM_MAX) {
             const int R = (int)((nr + 31) & ~31);
             int nt = 32 + (R <= 128 ? 4 * R : R);   // the pivot warp + the update warps
@@ -896,8 +903,9 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             int nt = 32 + (R <= 128 ? 4 * R : R);
             if (nt > 640) nt = 640;
             prof.begin(s, PROF_LU, fm * D.bs_lu_flops[(size_t)lv], D.bs_lu_bytes[(size_t)lv] * (double)vs);
-            if ((N.lu_variant & 3) == 1)
-                k_bat_lu5<T><<<cnt, LU5_THREADS, front_lu5_smem(D.bs_maxnr[(size_t)lv], D.bs_maxnp[(size_t)lv], vs), s>>>(
+            if ((N.lu_variant & 3) == 2)
+                k_bat_lu6<T><<<cnt, front_lu6_threads(D.bs_maxnr[(size_t)lv], D.bs_maxnp[(size_t)lv]),
+                               front_lu6_smem(D.bs_maxnr[(size_t)lv], D.bs_maxnp[(size_t)lv], vs), s>>>(
                     D.fc, bl, Wb, N.colmax, pivot_rel, N.rowid, La, N.permall, N.p_lu, N.st), note_launch();
             else
                 k_bat_lu2<T><<<cnt, nt, front_lu_smem(D.bs_maxnr[(size_t)lv], D.bs_maxnp[(size_t)lv], vs), s>>>(
