@@ -450,7 +450,9 @@ extern "C" int fplus_b200_graph_create(int64_t count, fplus_numeric *const *nums
         CKH(cudaMalloc(&b, bytes > 0 ? bytes : 16));
         g->rhs.push_back(b);
         CKH(cudaMemsetAsync(b, 0, bytes, N.stream));
+        N.capture_size = 1;
         rc = dev_solve(*num->plan, *num->dplan, N, b, nrhs[k], trans, err, errlen);
+        N.capture_size = 0;
         if (rc == FPLUS_OK) CKH(cudaStreamSynchronize(N.stream));
         cudaEvent_t e = nullptr;
         CKH(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

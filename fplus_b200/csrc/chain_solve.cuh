@@ -1,5 +1,5 @@
 // chain_solve.cuh -- the triangular sweeps through the dense chain (fronts of at most 64 pivots whose columns are all of
-// [f, n), each front's contribution block the next one's only child).
+// [f, n), each front's contribution block the next one's only child), and the packed triangles that all sweeps read.
 //
 // The chain is one dependency: K blocks of nb unknowns, each needing every one before it.  The column sweeps (U, U^T) read
 // n^2 / 2 entries of U12 (8.6 GB for n = 32,768 complex), the row sweeps (L, L^T) K blocks of at most 256 x 64.
@@ -9,72 +9,131 @@
 //              these appear, two or more blocks ahead of the solver (which takes the product with the block just solved
 //              itself, from shared memory).  U12's 64 x 64 blocks are contiguous and stream through a ring of shared
 //              memory without waiting for x.  Cross-CTA order: a counter of the blocks solved and a flag per block whose
-//              products are all in, release / acquire, waits bounded.  A cooperative launch, so all CTAs are resident.
+//              products are all in, release / acquire, waits bounded.  All CTAs are resident together: one cluster, or a
+//              cooperative launch.
 //   k_chain_l  L (TR 0) or L^T (TR 1, 2) by one CTA per group of right-hand sides, the front's row vector in shared
 //              memory from front to front (no global round trip), L streamed in 16-column pieces.
-// Both solve a front's triangle by 16 x 16 diagonal blocks inverted once per factorization (k_chain_dinv): four dependent
-// products instead of 64 dependent steps.
+// Both solve a front's triangle by 16 x 16 diagonal blocks inverted once per factorization: four dependent products instead
+// of 64 dependent steps.  All streams are bulk copies (cp.async.bulk) of contiguous, packed pieces: element-wise cp.async
+// issued 26 cycles a warp and held the shared-memory loads of the chain up behind it (a 16 x 16 product took 2,800 cycles).
 #pragma once
 #include "kernels.cuh"
 
 namespace fpl {
 
-constexpr int CH_THREADS = 256, CH_NB = 64, CH_MAXNR = 256, CH_STAGES = 3;
-constexpr unsigned CH_SPIN = 1u << 22;          // polls before a wait gives up (about a second)
+constexpr int CH_THREADS = 256, CH_NB = 64, CH_MAXNR = 256, CH_STAGES = 3, CH_UTHREADS = CH_THREADS + 64;
+constexpr unsigned CH_SPIN = 1u << 22;          // polls before a wait for another CTA gives up (about a second)
+constexpr long long CH_CYCLES = 4000000000ll;   // the longest wait for a bulk copy (about two seconds)
+constexpr int CH_BLK = CH_NB * CH_NB + 2;       // a ring stage (two elements more: see chain_ublock)
 
 // a chain front as the sweeps read it; nslot, slot, tau: where the previous chain front's contribution rows enter (its row t
-// at initial row slot + t, t < nslot, or tau + t - nslot)
+// at initial row slot + t, t < nslot, or tau + t - nslot); u_pk, l_pk: its packed pieces
 struct ChainFront {
-    long long f, np, nr, L_off, U_off, row_off, nslot, slot, tau;
+    long long f, np, nr, row_off, nslot, slot, tau, u_pk, l_pk;
 };
 
-// the inverses of the 16 x 16 diagonal blocks of a chain front's U11 (dinv[0 .. 4)) and unit-lower L11 (dinv[4 .. 8)),
-// column-major, identity beyond the front's pivots; a thread per column
+// Packed pieces of a front's triangles, one per 16 pivots (block b, k0 = 16 b): the inverted diagonal block (256 elements,
+// column-major, identity beyond the front's pivots), then the 16 columns' other entries (zero beyond the pivots):
+//   U piece b: rows [0, k0) of U11's columns (leading dimension k0), at u_pk + pk_u(b)
+//   L piece b: rows [k0 + w, R) of L's columns (w pivots in the block, leading dimension R - k0 - w), at l_pk + pk_l(b, R);
+//              R = the front's rows on the dense chain, its pivots elsewhere
+__host__ __device__ constexpr int64_t pk_u(int64_t b) { return 256 * b + 128 * b * (b - 1); }
+__host__ __device__ constexpr int64_t pk_l(int64_t b, int64_t R) { return 256 * b + 16 * b * R - 128 * b * (b + 1); }
+
 template <typename T>
-__global__ void __launch_bounds__(128) k_chain_dinv(const ChainFront *__restrict__ fr, const T *__restrict__ La, T *__restrict__ dinv,
-                                                    const DevStatus *st)
+__global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ fr, const int *__restrict__ dfront, const T *__restrict__ La,
+                                                    T *__restrict__ pk, const DevStatus *st)
 {
     if (st->code) return;
-    const ChainFront F = fr[blockIdx.x];
-    const int lower = threadIdx.x >> 6, b = (threadIdx.x >> 4) & 3, c = threadIdx.x & 15;
-    const int np = (int)F.np, k0 = 16 * b;
+    const int64_t blk = blockIdx.x;
+    const SvFront F = fr[dfront[blk]];
+    const int np = (int)(F.np < F.nr ? F.np : F.nr), b = (int)(blk - F.d_off), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const T *L = La + F.L_off;
-    T x[16];
-    auto at = [&](int i, int k) -> T { return k0 + i < np && k0 + k < np ? L[(k0 + i) + (int64_t)(k0 + k) * F.nr] : VT<T>::zero(); };
-    if (lower) {
+    T *du = pk + F.u_pk + pk_u(b), *dl = pk + F.l_pk + pk_l(b, F.l_rows);
+    if (warp == 0) {                                    // the inverses: a lane per column (U's, then L's)
+        const int lower = lane >> 4, c = lane & 15;
+        T x[16];
+        auto at = [&](int i, int k) -> T { return k0 + i < np && k0 + k < np ? L[(k0 + i) + (int64_t)(k0 + k) * F.nr] : VT<T>::zero(); };
+        if (lower) {
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            T s = i == c ? VT<T>::one() : VT<T>::zero();
+            for (int i = 0; i < 16; i++) {
+                T s = i == c ? VT<T>::one() : VT<T>::zero();
 #pragma unroll
-            for (int k = 0; k < i; k++) s = msub(s, at(i, k), x[k]);
-            x[i] = s;
+                for (int k = 0; k < i; k++) s = msub(s, at(i, k), x[k]);
+                x[i] = s;
+            }
+        } else {
+#pragma unroll
+            for (int i = 15; i >= 0; i--) {
+                T s = i == c ? VT<T>::one() : VT<T>::zero();
+#pragma unroll
+                for (int k = 15; k > i; k--) s = msub(s, at(i, k), x[k]);
+                const T d = at(i, i);                   // (never zero: the factorization reports such a column as singular)
+                x[i] = k0 + i < np ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
+            }
         }
-    } else {
+        T *o = (lower ? dl : du) + c * 16;
 #pragma unroll
-        for (int i = 15; i >= 0; i--) {
-            T s = i == c ? VT<T>::one() : VT<T>::zero();
-#pragma unroll
-            for (int k = 15; k > i; k--) s = msub(s, at(i, k), x[k]);
-            const T d = at(i, i);
-            x[i] = k0 + i < np ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
-        }
+        for (int i = 0; i < 16; i++) o[i] = x[i];
     }
-    T *o = dinv + ((int64_t)blockIdx.x * 8 + 4 * lower + b) * 256 + c * 16;
-#pragma unroll
-    for (int i = 0; i < 16; i++) o[i] = x[i];
+    const int rl = (int)F.l_rows - k0 - w;
+    for (int c = warp; c < 16; c += 4) {
+        const bool in = c < w;
+        const T *src = L + (int64_t)(k0 + (in ? c : 0)) * F.nr;
+        for (int r = lane; r < k0; r += 32) du[256 + c * k0 + r] = in ? src[r] : VT<T>::zero();
+        for (int r = lane; r < rl; r += 32) dl[256 + c * rl + r] = in ? src[k0 + w + r] : VT<T>::zero();
+    }
 }
 
-template <int N> __device__ __forceinline__ void cp_async_wait_n() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned long long *bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+// a bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned) that completes on `bar`
+__device__ __forceinline__ void bulk_expect(unsigned long long *bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool bar_try(unsigned long long *bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// waits for the phase; false when the wait ran out of time
+__device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity)
+{
+    if (bar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!bar_try(bar, parity))
+        if (clock64() - t0 > CH_CYCLES) return false;
+    return true;
+}
+
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// one thread waits until *p >= v; false when the wait ran out
+// arrive at a named barrier without waiting
+__device__ __forceinline__ void named_arrive(int id, int count) { asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+// one thread waits until *p >= v; false when the wait ran out.  It polls with relaxed loads (an acquiring load each time
+// invalidates the SM's L1, which slowed the other warps' products threefold) and acquires once
 __device__ __forceinline__ bool chain_wait(const unsigned *p, unsigned v)
 {
-    for (unsigned k = 0; k < CH_SPIN; k++)
-        if (ld_acquire_u32(p) >= v) return true;
+    for (unsigned k = 0; k < CH_SPIN; k++) {
+        unsigned c;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(p) : "memory");
+        if (c >= v) { (void)ld_acquire_u32(p); return true; }
+        __nanosleep(20);
+    }
     return false;
 }
 template <typename T> __device__ __forceinline__ T madd(T a, T l, T p);
@@ -86,373 +145,577 @@ template <> __device__ __forceinline__ cplx madd<cplx>(cplx a, cplx l, cplx p)
 template <int TR> __device__ __forceinline__ double opv(double v) { return v; }
 template <int TR> __device__ __forceinline__ cplx opv(cplx v) { return TR == 2 ? cplx{v.x, -v.y} : v; }
 
-// acc[r] = sum over this lane's share of the inner index k < kn of M(o, k) x[k + r * xld], four lanes (q) per output o,
-// then summed over the four lanes.  M(o, k) = Mp[k * ld + o] (plain), or op(Mp[o * ld + k]) (transposed; the lanes of
-// neighbouring outputs start two apart, so that they read other banks)
+// The sum over k < kn (a multiple of 16) of M(o, k) x[k * RB + r] by four lanes per output, each with four of every sixteen k,
+// then summed over the four lanes.  The output o and the lane's share q of thread tid (a warp: eight outputs, lane = o + 8 q,
+// so that the eight lanes of a shared-memory phase read eight neighbouring elements: with the shares in neighbouring lanes a
+// 64 x 64 product took 2,700 cycles).  M(o, k) = Mp[k * ld + o] (plain), or op(Mp[o * ld + k]) (transposed; neighbouring
+// outputs start one apart)
+__device__ __forceinline__ int quad_o(int tid) { return (tid & 7) + 8 * (tid >> 5); }
+__device__ __forceinline__ int quad_q(int tid) { return (tid >> 3) & 3; }
+template <typename T, int RB> __device__ __forceinline__ void quad_sum(T (&acc)[RB])
+{
+#pragma unroll
+    for (int r = 0; r < RB; r++) {
+        acc[r] = add(acc[r], shfl_xor_v<T>(acc[r], 8));
+        acc[r] = add(acc[r], shfl_xor_v<T>(acc[r], 16));
+    }
+}
 template <typename T, int TR, int RB>
-__device__ __forceinline__ void quad_mv(T (&acc)[RB], const T *Mp, int ld, int o, int q, int kn, const T *x, int xld, int rb)
+__device__ __forceinline__ void quad_mv(T (&acc)[RB], const T *Mp, int ld, int o, int q, int kn, const T *x)
 {
 #pragma unroll
     for (int r = 0; r < RB; r++) acc[r] = VT<T>::zero();
-    const int ne = (kn + 3) >> 2;
-#pragma unroll 4
-    for (int e = 0; e < ne; e++) {
-        int k;
-        if (TR == 0) k = q + 4 * e;
-        else { int ee = e + (o & 1); if (ee >= ne) ee -= ne; k = q + 4 * ee; }
-        if (k < kn) {
-            const T m = TR == 0 ? Mp[k * ld + o] : opv<TR>(Mp[o * ld + k]);
+    const T *m = TR == 0 ? Mp + q * ld + o : Mp + o * ld;
+    const int ms = 4 * ld;
+    for (int e = 0; e < kn; e += 16) {
+        T v[4];
+        int k[4];
 #pragma unroll
-            for (int r = 0; r < RB; r++) if (r < rb) acc[r] = madd<T>(acc[r], m, x[k + r * xld]);
+        for (int z = 0; z < 4; z++) {
+            k[z] = TR == 0 ? e + q + 4 * z : e + ((4 * q + z + o) & 15);
+            v[z] = TR == 0 ? m[z * ms] : opv<TR>(m[k[z]]);
         }
-    }
+        if (TR == 0) m += 4 * ms;
 #pragma unroll
-    for (int r = 0; r < RB; r++) {
-        acc[r] = add(acc[r], shfl_xor_v<T>(acc[r], 1));
-        acc[r] = add(acc[r], shfl_xor_v<T>(acc[r], 2));
+        for (int z = 0; z < 4; z++)
+#pragma unroll
+            for (int r = 0; r < RB; r++) acc[r] = madd<T>(acc[r], v[z], x[k[z] * RB + r]);
     }
+    quad_sum<T, RB>(acc);
 }
 
-// dynamic shared memory of k_chain_u for `own` blocks per worker and rb right-hand sides (the larger of the two roles)
+// right-hand sides per pass of the multiple-right-hand-side forms
+template <typename T> __host__ __device__ constexpr int ch_rb() { return VT<T>::cplx_ ? 4 : 8; }
+// dynamic shared memory of k_chain_u for `own` blocks' sums per worker (the larger of the two roles)
 static inline size_t chain_u_smem(int64_t own, int64_t rb, int64_t vs)
 {
-    const size_t worker = (size_t)(CH_STAGES * CH_NB * CH_NB + CH_NB * rb * (1 + own)) * vs;
-    const size_t solver = (size_t)(2 * CH_NB * CH_NB + 2 * 2560 + 2 * CH_NB * rb) * vs;
+    const size_t worker = (size_t)(CH_STAGES * CH_BLK + CH_NB * rb * (1 + own)) * vs;
+    const size_t solver = (size_t)(2 * CH_BLK + 2 * 2560 + 4 * CH_NB * rb) * vs;
     return worker > solver ? worker : solver;
 }
 
-// t = 0 .. K - 1: the blocks in solve order (TR 0: front K - 1 - t, else front t).  Y: the right-hand sides (pivot order,
-// overwritten), X: the solution; both n x nrhs.  sync[0]: blocks solved; sync[1 + t]: block t has every product but that of
-// block t - 1.  RB >= rb right-hand sides.
+// x = U11^-1 y (TR 0) or U11^-T y of one chain front from its packed pieces tr, by CH_THREADS threads (o, q: quad_o, quad_q;
+// ys and x: [k * RB + r], zero beyond the pivots; ys is overwritten); ends without a barrier after the last writes of x but
+// the named barrier 1 of its steps
 template <typename T, int TR, int RB>
-__global__ void __launch_bounds__(CH_THREADS) k_chain_u(const ChainFront *__restrict__ fr, int K, int nb, const T *__restrict__ La,
-                                                        const T *__restrict__ Ua, const T *__restrict__ dinv, T *Y, T *X, int64_t n,
-                                                        int rb, unsigned *sync, DevStatus *st)
+__device__ __forceinline__ void chain_tri(const T *tr, T *ys, T *x, int nbk, int o, int q)
+{
+    T a[RB];
+    for (int bb = 0; bb < nbk; bb++) {
+        const int b = TR == 0 ? nbk - 1 - bb : bb, k0 = 16 * b;
+        const T *D = tr + pk_u(b), *pan = D + 256;         // (16 columns, leading dimension k0)
+        if (TR != 0 && b > 0) {
+            // w_b -= U[0 .. 16b, b]^T z
+            if (o < 16) {
+                quad_mv<T, TR, RB>(a, pan, k0, o, q, k0, x);
+                if (q == 0)
+#pragma unroll
+                    for (int r = 0; r < RB; r++) ys[(k0 + o) * RB + r] = sub(ys[(k0 + o) * RB + r], a[r]);
+            }
+            named_bar(1, CH_THREADS);
+        }
+        if (o < 16) {                              // (beyond the pivots: identity times zero)
+            quad_mv<T, TR, RB>(a, D, 16, o, q, 16, ys + k0 * RB);
+            if (q == 0)
+#pragma unroll
+                for (int r = 0; r < RB; r++) x[(k0 + o) * RB + r] = a[r];
+        }
+        named_bar(1, CH_THREADS);
+        if (TR == 0 && b > 0) {
+            // y[0 .. 16b) -= U[0 .. 16b, b] x_b
+            if (o < k0) {
+                quad_mv<T, 0, RB>(a, pan, k0, o, q, 16, x + k0 * RB);
+                if (q == 0)
+#pragma unroll
+                    for (int r = 0; r < RB; r++) ys[o * RB + r] = sub(ys[o * RB + r], a[r]);
+            }
+            named_bar(1, CH_THREADS);
+        }
+    }
+}
+
+// the product of a 64 x 64 block with the kn values of xs (quad_mv, the last front's odd lengths included); oo: this
+// thread's output, or 0 beyond the outputs
+template <typename T, int TR, int RB>
+__device__ __forceinline__ void block_mv(T (&a)[RB], const T *M, int nb, int oo, int q, int kn, const T *xs)
+{
+    if ((kn & 15) == 0) { quad_mv<T, TR, RB>(a, M, nb, oo, q, kn, xs); return; }
+#pragma unroll
+    for (int r = 0; r < RB; r++) a[r] = VT<T>::zero();
+    for (int k = q; k < kn; k += 4) {
+        const T m = TR == 0 ? M[k * nb + oo] : opv<TR>(M[oo * nb + k]);
+#pragma unroll
+        for (int r = 0; r < RB; r++) a[r] = madd<T>(a[r], m, xs[k * RB + r]);
+    }
+    quad_sum<T, RB>(a);
+}
+
+// t = 0 .. K - 1: the blocks in solve order (TR 0: front K - 1 - t, else front t); front k's pivots are [f0 + k nb, ..) and
+// its U12 starts at U0 + sum of the fronts' before it.  Y: the right-hand sides (pivot order, overwritten), X: the
+// solution; both n x nrhs.  sync[0]: blocks solved; sync[1 + t]: block t has every product but that of block t - 1.
+// rb <= RB right-hand sides.
+//
+// What bounds it: at small K the solver's step (the 64 x 64 product with the block just solved, then four 16 x 16 products
+// and their updates) and the round trip solver - worker - solver; at large K the stream of U12.
+template <typename T, int TR, int RB>
+__global__ void __launch_bounds__(CH_UTHREADS) k_chain_u(const ChainFront *__restrict__ fr, int K, int nb, int64_t f0, int64_t U0,
+                                                         int np_last, const T *__restrict__ Ua, const T *__restrict__ pk, T *Y, T *X,
+                                                         int64_t n, int rb, unsigned *sync, T *gacc, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned long long bars[CH_STAGES];
     __shared__ int s_ok;
-    const int tid = threadIdx.x, o = tid >> 2, q = tid & 3;
+    const int tid = threadIdx.x, o = quad_o(tid), q = quad_q(tid);
     auto front_of = [&](int t) -> int { return TR == 0 ? K - 1 - t : t; };
-    const int np_last = (int)fr[K - 1].np;
     auto np_of = [&](int t) -> int { return front_of(t) == K - 1 ? np_last : nb; };
-    // the 64 x 64 block of U12 that couples block t to block s < t in solve order, and its column count
-    auto block_ptr = [&](int t, int s) -> const T * {
-        const int a = TR == 0 ? front_of(t) : front_of(s), c = TR == 0 ? front_of(s) : front_of(t);    // rows of front a, columns of front c > a
-        return Ua + fr[a].U_off + (int64_t)(c - a - 1) * nb * nb;
+    auto f_of = [&](int t) -> int64_t { return f0 + (int64_t)front_of(t) * nb; };
+    // the block of U12 that couples block t to block s < t in solve order (rows of front a, columns of front c > a); where
+    // its start is not 16-byte aligned the copy takes one element more before and after it, and sh is 1
+    const int sh = VT<T>::cplx_ ? 0 : (int)(U0 & 1);
+    auto load_block = [&](T *dst, int t, int s, unsigned long long *bar) {
+        const int a = TR == 0 ? front_of(t) : front_of(s), c = TR == 0 ? front_of(s) : front_of(t);
+        const int64_t off = U0 + (int64_t)nb * ((int64_t)a * (n - f0) - (int64_t)nb * a * (a + 1) / 2) + (int64_t)(c - a - 1) * nb * nb;
+        const int cnt = nb * (c == K - 1 ? np_last : nb);
+        // (an odd count of 8-byte elements, in the last front only, is rounded up: the arena has room behind it)
+        const unsigned bytes = (unsigned)((((size_t)(cnt + 2 * sh) * sizeof(T)) + 15) & ~(size_t)15);
+        bulk_expect(bar, bytes);
+        bulk_load(dst, Ua + off - sh, bytes, bar);
     };
-    auto block_size = [&](int t, int s) -> int { return nb * (TR == 0 ? np_of(s) : np_of(t)); };
-    auto copy = [&](T *dst, const T *src, int cnt) { for (int e = tid; e < cnt; e += CH_THREADS) cp_async_el(dst + e, src + e); };
-    if (st->code) return;
+    if (tid == 0) {
+        s_ok = st->code == 0;
+        for (int k = 0; k < CH_STAGES; k++) bar_init(bars + k, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (!*(volatile int *)&s_ok) return;
     if (blockIdx.x > 0) {
+        if (tid >= CH_THREADS) return;                 // (the solver's helper warps)
         // a worker: owns the blocks t = w, w + W, .. (w = blockIdx.x - 1)
         const int w = blockIdx.x - 1, W = gridDim.x - 1;
         T *ring = reinterpret_cast<T *>(smem_raw);
-        T *xs = ring + CH_STAGES * CH_NB * CH_NB;      // x of the block being subtracted: xs[k + r * CH_NB]
-        T *acc = xs + CH_NB * rb;                      // owned block j's sums: acc[(j * rb + r) * CH_NB + o]
+        T *xs = ring + CH_STAGES * CH_BLK;             // x of the block being subtracted: xs[k * RB + r]
+        // owned block j's sums, in shared memory (after x), or in global memory (gacc, block t's at t): [o * RB + r] from
+        // acc + j * ajs on; each entry is its thread's own
         const int own = w < K ? (K - 1 - w) / W + 1 : 0;
-        for (int e = tid; e < own * rb * CH_NB; e += CH_THREADS) acc[e] = VT<T>::zero();
-        // tasks in order: s ascending, the owned t >= s + 2 ascending
-        auto first_t = [&](int s) -> int { const int m = s + 2; return m <= w ? w : w + (m - w + W - 1) / W * W; };
-        int ps = 0, pt = 0;                            // the next task to load
-        auto settle = [&](int &s, int &t) { while (s <= K - 3 && t >= K) { s++; t = first_t(s); } };
-        pt = first_t(0);
-        settle(ps, pt);
-        int cs = ps, ct = pt;                          // the task to compute
-        auto load_next = [&](int slot) {
+        T *acc = gacc ? gacc + (int64_t)w * CH_NB * RB : xs + CH_NB * RB;
+        const int64_t ajs = (gacc ? (int64_t)W : 1) * CH_NB * RB;
+        if (q == 0) for (int j = 0; j < own; j++)
+#pragma unroll
+            for (int r = 0; r < RB; r++) acc[j * ajs + o * RB + r] = VT<T>::zero();
+        for (int e = tid; e < RB * CH_NB; e += CH_THREADS) xs[e] = VT<T>::zero();
+        // tasks in order: s ascending, the owned t >= s + 2 ascending (t = w + j W, j from j0(s))
+        auto first_j = [&](int s) -> int { const int m = s + 2 - w; return m <= 0 ? 0 : (m + W - 1) / W; };
+        int ps = 0, pj = first_j(0), cs, cj, issued = 0, done = 0;
+        while (ps <= K - 3 && pj >= own) { ps++; pj = first_j(ps); }
+        cs = ps; cj = pj;
+        auto load_next = [&]() {                       // one thread
             if (ps <= K - 3) {
-                copy(ring + slot * CH_NB * CH_NB, block_ptr(pt, ps), block_size(pt, ps));
-                pt += W;
-                settle(ps, pt);
+                load_block(ring + (issued % CH_STAGES) * CH_BLK, w + pj * W, ps, bars + issued % CH_STAGES);
+                issued++;
+                pj++;
+                while (ps <= K - 3 && pj >= own) { ps++; pj = first_j(ps); }
             }
-            cp_async_commit();
         };
-        for (int k = 0; k < CH_STAGES - 1; k++) load_next(k);
-        int slot = 0, have = -1;
+        if (tid == CH_THREADS - 1) for (int k = 0; k < CH_STAGES; k++) load_next();
+        int have = -1;
         while (cs <= K - 3) {
             if (have != cs) {                          // a new solved block: wait for it, its x into shared memory
-                if (tid == 0) s_ok = chain_wait(sync, (unsigned)cs + 1u);
-                __syncthreads();
-                if (!s_ok) { if (tid == 0) set_status(st, ST_WAIT, cs, 0, 0); break; }
-                const int64_t f = fr[front_of(cs)].f;
+                if (tid == 0 && !chain_wait(sync, (unsigned)cs + 1u)) s_ok = 0;
+                named_bar(1, CH_THREADS);
+                const int64_t f = f_of(cs);
                 const int np = np_of(cs);
-                for (int e = tid; e < np * rb; e += CH_THREADS) { const int k = e % np, r = e / np; xs[k + r * CH_NB] = ldcg_v(X + f + k + r * n); }
+                if (*(volatile int *)&s_ok)
+                    for (int e = tid; e < CH_NB * rb; e += CH_THREADS) {
+                        const int k = e & (CH_NB - 1), r = e / CH_NB;
+                        xs[k * RB + r] = k < np ? ldcg_v(X + f + k + r * n) : VT<T>::zero();
+                    }
                 have = cs;
+                named_bar(1, CH_THREADS);
             }
-            cp_async_wait_n<CH_STAGES - 2>();
-            __syncthreads();                           // the block and x are in; the slot before is free
-            load_next((slot + CH_STAGES - 1) % CH_STAGES);
-            const int no = TR == 0 ? nb : np_of(ct), kn = TR == 0 ? np_of(cs) : nb;
+            const int slot = done % CH_STAGES, ct = w + cj * W;
+            if (!bar_wait(bars + slot, (unsigned)(done / CH_STAGES) & 1u)) s_ok = 0;
+            const int no = TR == 0 ? nb : np_of(ct);
+            // (the inner length in whole sixteens: x is zero beyond the block; nb is one, and so are U12's columns but in the
+            // last front, whose block's copy may hold less: those columns are not read)
+            const int kn = TR == 0 ? np_of(cs) : nb;
             T a[RB];
-            quad_mv<T, TR, RB>(a, ring + slot * CH_NB * CH_NB, nb, o < no ? o : 0, q, kn, xs, CH_NB, rb);
-            T *ao = acc + (int64_t)((ct - w) / W) * rb * CH_NB + o;
+            const T *M = ring + slot * CH_BLK + sh;
+            block_mv<T, TR, RB>(a, M, nb, o < no ? o : 0, q, kn, xs);
+            T *ao = acc + cj * ajs + o * RB;
+            const bool last = cs == ct - 2;            // the last product this worker takes for block ct
             if (q == 0 && o < no) {
 #pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) ao[r * CH_NB] = add(ao[r * CH_NB], a[r]);
-                if (cs == ct - 2) {                    // the last product this worker takes for block ct
-                    T *y = Y + fr[front_of(ct)].f + o;
+                for (int r = 0; r < RB; r++) a[r] = add(ao[r], a[r]);
+                if (last) {
+                    T *y = Y + f_of(ct) + o;
 #pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rb) y[r * n] = sub(y[r * n], ao[r * CH_NB]);
+                    for (int r = 0; r < RB; r++) if (r < rb) y[r * n] = sub(y[r * n], a[r]);
                     __threadfence();
+                } else {
+#pragma unroll
+                    for (int r = 0; r < RB; r++) ao[r] = a[r];
                 }
             }
-            if (cs == ct - 2) {
-                __syncthreads();
-                if (tid == 0) st_release_u32(sync + 1 + ct, 1u);
-            }
-            slot = (slot + 1) % CH_STAGES;
-            ct += W;
-            settle(cs, ct);
+            named_bar(1, CH_THREADS);                  // the stage is free, the sums are out
+            if (!*(volatile int *)&s_ok) { if (tid == 0) set_status(st, ST_WAIT, cs, 0, 0); break; }
+            if (last && tid == 0) st_release_u32(sync + 1 + ct, 1u);
+            if (tid == CH_THREADS - 1) load_next();
+            done++;
+            cj++;
+            while (cs <= K - 3 && cj >= own) { cs++; cj = first_j(cs); }
         }
-        cp_async_wait_n<0>();
+        // the copies in flight (after a wait that ran out)
+        if (tid == CH_THREADS - 1) for (; done < issued; done++) (void)bar_wait(bars + done % CH_STAGES, (unsigned)(done / CH_STAGES) & 1u);
         return;
     }
-    // the solver
+    // the solver: 256 threads on the critical path and two helper warps, one that waits for the workers' part of the next
+    // block's right-hand side and brings it in, one that publishes the solved block (the stores, the fence, the counter)
     T *off = reinterpret_cast<T *>(smem_raw);          // two stages: the block coupling t to t - 1
-    T *tri = off + 2 * CH_NB * CH_NB;                  // two stages: U11's 16-column panels above the diagonal blocks (panel b: 16b rows,
-                                                       // at 256 b (b - 1) / 2), then the four inverted diagonal blocks (at 1536)
-    T *ys = tri + 2 * 2560, *xs = ys + CH_NB * rb;
+    T *tri = off + 2 * CH_BLK;                         // two stages: the front's packed U pieces
+    T *yin = tri + 2 * 2560, *xs = yin + 2 * CH_NB * RB;       // right-hand sides and solutions, two blocks each in turn: [k * RB + r]
+    for (int e = tid; e < 4 * CH_NB * RB; e += CH_UTHREADS) yin[e] = VT<T>::zero();
+    __syncthreads();
+    if (tid >= CH_THREADS) {
+        const int lane = tid & 31;
+        if (tid < CH_THREADS + 32) {                   // right-hand sides in
+            for (int t = 0; t < K; t++) {
+                const int np = np_of(t);
+                int ok = 1;
+                if (t >= 2 && lane == 0) ok = chain_wait(sync + 1 + t, 1u);
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                const int64_t f = f_of(t);
+                if (ok) for (int e = lane; e < CH_NB * rb; e += 32) {
+                    const int p = e & (CH_NB - 1), r = e / CH_NB;
+                    yin[((t & 1) * CH_NB + p) * RB + r] = p < np ? ldcg_v(Y + f + p + r * n) : VT<T>::zero();
+                }
+                else if (lane == 0) { set_status(st, ST_WAIT, t, 0, 0); s_ok = 0; }
+                __syncwarp();
+                named_bar(3, CH_THREADS + 32);         // block t's right-hand side is in
+                if (!*(volatile int *)&s_ok) return;
+            }
+        } else {                                       // solved blocks out
+            for (int t = 0; t < K; t++) {
+                named_bar(4 + (t & 1), CH_THREADS + 32);       // block t is solved (or a wait ran out)
+                if (!*(volatile int *)&s_ok) return;
+                const int np = np_of(t);
+                const int64_t f = f_of(t);
+                for (int e = lane; e < np * rb; e += 32) { const int p = e % np, r = e / np; X[f + p + r * n] = xs[((t & 1) * CH_NB + p) * RB + r]; }
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) st_release_u32(sync, (unsigned)t + 1u);
+            }
+        }
+        return;
+    }
+    long long upk = tid == CH_THREADS - 1 ? fr[front_of(0)].u_pk : 0;      // the loading thread: the next block's packed pieces
     auto load = [&](int t) {
         if (t < K) {
-            const int sl = t & 1, k = front_of(t), np = np_of(t);
-            T *tr = tri + sl * 2560;
-            const T *L = La + fr[k].L_off;
-            const int64_t nr = fr[k].nr;
-            if (t > 0) copy(off + sl * CH_NB * CH_NB, block_ptr(t, t - 1), block_size(t, t - 1));
-            const T *dv = dinv + (int64_t)k * 8 * 256;
-            copy(tr + 1536, dv, 1024);
-            for (int e = tid; e < 1536; e += CH_THREADS) {
-                const int b = e < 256 ? 1 : e < 768 ? 2 : 3, p = e - 128 * b * (b - 1), rows = 16 * b, r = p % rows, c = 16 * b + p / rows;
-                if (c < np) cp_async_el(tr + e, L + r + (int64_t)c * nr);
-            }
+            const int sl = t & 1, np = np_of(t);
+            unsigned long long *bar = bars + sl;
+            const unsigned bytes = (unsigned)(pk_u((np + 15) >> 4) * sizeof(T));
+            if (t > 0) {
+                const int s = t - 1, a = TR == 0 ? front_of(t) : front_of(s), c = TR == 0 ? front_of(s) : front_of(t);
+                const int64_t uo = U0 + (int64_t)nb * ((int64_t)a * (n - f0) - (int64_t)nb * a * (a + 1) / 2);
+                const unsigned ub = (unsigned)((((size_t)(nb * (c == K - 1 ? np_last : nb) + 2 * sh) * sizeof(T)) + 15) & ~(size_t)15);
+                bulk_expect(bar, bytes + ub);
+                bulk_load(off + sl * CH_BLK, Ua + uo - sh, ub, bar);
+            } else bulk_expect(bar, bytes);
+            bulk_load(tri + sl * 2560, pk + upk, bytes, bar);
+            if (t + 1 < K) upk = fr[front_of(t + 1)].u_pk;
         }
-        cp_async_commit();
     };
-    load(0);
+    if (tid == CH_THREADS - 1) load(0);
     for (int t = 0; t < K; t++) {
-        const int sl = t & 1, k = front_of(t), np = np_of(t), nbk = (np + 15) >> 4;
-        const int64_t f = fr[k].f;
-        if (tid == 0) s_ok = t < 2 || chain_wait(sync + 1 + t, 1u);
-        cp_async_wait_n<0>();
-        __syncthreads();
-        if (!s_ok) { if (tid == 0) set_status(st, ST_WAIT, t, 0, 0); break; }
-        load(t + 1);                                   // (into the stage that block t - 1 used)
+        const int sl = t & 1, np = np_of(t), nbk = (np + 15) >> 4;
+        T *ys = yin + sl * CH_NB * RB, *x = xs + sl * CH_NB * RB;
+        const T *xp = xs + (sl ^ 1) * CH_NB * RB;
+        if (tid == CH_THREADS - 1) load(t + 1);        // (into the stage that block t - 1 used: everyone is past it)
+        if (!bar_wait(bars + sl, (unsigned)(t >> 1) & 1u)) { set_status(st, ST_WAIT, t, 0, 0); s_ok = 0; }
+        named_bar(3, CH_THREADS + 32);                 // the copies, and the right-hand side
+        if (!*(volatile int *)&s_ok) {
+            // (the copies in flight land first)
+            if (tid == CH_THREADS - 1) { (void)bar_wait(bars + sl, (unsigned)(t >> 1) & 1u); if (t + 1 < K) (void)bar_wait(bars + (sl ^ 1), (unsigned)((t + 1) >> 1) & 1u); }
+            named_bar(4 + (t & 1), CH_THREADS + 32);
+            break;
+        }
         T a[RB];
-        if (t > 0) quad_mv<T, TR, RB>(a, off + sl * CH_NB * CH_NB, nb, o < np ? o : 0, q, np_of(t - 1), xs, CH_NB, rb);
-        if (q == 0 && o < np) {
-            const T d = La[fr[k].L_off + o + (int64_t)o * fr[k].nr];
-            if (is_zero(d)) set_status(st, ST_SOLVE_ZERO, f + o, 0, 0);
+        if (t > 0) {
+            const int kn = np_of(t - 1);
+            const T *M = off + sl * CH_BLK + sh;
+            block_mv<T, TR, RB>(a, M, nb, o < np ? o : 0, q, kn, xp);
+            if (q == 0 && o < np)
 #pragma unroll
-            for (int r = 0; r < RB; r++)
-                if (r < rb) {
-                    const T y = ldcg_v(Y + f + o + r * n);
-                    ys[o + r * CH_NB] = t > 0 ? sub(y, a[r]) : y;
-                }
+                for (int r = 0; r < RB; r++) ys[o * RB + r] = sub(ys[o * RB + r], a[r]);
         }
-        __syncthreads();
-        const T *tr = tri + sl * 2560;
-        for (int bb = 0; bb < nbk; bb++) {
-            const int b = TR == 0 ? nbk - 1 - bb : bb, k0 = 16 * b;
-            const T *pan = tr + 128 * b * (b - 1);     // panel b (16b rows)
-            if (TR != 0 && b > 0) {
-                // w_b -= U[0 .. 16b, b]^T z
-                if (o < 16) {
-                    quad_mv<T, TR, RB>(a, pan, 16 * b, k0 + o < np ? o : 0, q, k0, xs, CH_NB, rb);
-                    if (q == 0 && k0 + o < np)
-#pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rb) ys[k0 + o + r * CH_NB] = sub(ys[k0 + o + r * CH_NB], a[r]);
-                }
-                __syncthreads();
-            }
-            const int w16 = np - k0 < 16 ? np - k0 : 16;
-            if (o < 16) {
-                quad_mv<T, TR, RB>(a, tr + 1536 + 256 * b, 16, o < w16 ? o : 0, q, w16, ys + k0, CH_NB, rb);
-                if (q == 0 && o < w16)
-#pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rb) { xs[k0 + o + r * CH_NB] = a[r]; X[f + k0 + o + r * n] = a[r]; }
-            }
-            __syncthreads();
-            if (TR == 0 && b > 0) {
-                // y[0 .. 16b) -= U[0 .. 16b, b] x_b
-                if (o < k0) {
-                    quad_mv<T, 0, RB>(a, pan, 16 * b, o, q, w16, xs + k0, CH_NB, rb);
-                    if (q == 0)
-#pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rb) ys[o + r * CH_NB] = sub(ys[o + r * CH_NB], a[r]);
-                }
-                __syncthreads();
-            }
-        }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) st_release_u32(sync, (unsigned)t + 1u);
+        named_bar(1, CH_THREADS);
+        chain_tri<T, TR, RB>(tri + sl * 2560, ys, x, nbk, o, q);
+        named_arrive(4 + (t & 1), CH_THREADS + 32);    // x is in shared memory: out it goes (two barriers in turn: block t + 2
+                                                       // cannot be done before block t is out)
     }
-    cp_async_wait_n<0>();
 }
 
-// dynamic shared memory of k_chain_l: CH_LSTAGES pieces of 16 columns (with the inverted diagonal block), two row vectors
+// One step of the same sweep as a launch of its own (s = -1 .. K - 2): CTA 0 solves block s + 1, the others add the product
+// with block s to the sums of the blocks from s + 2 on (gacc: block t's at t CH_NB RB).  Every value is formed as k_chain_u
+// forms it, so the results are the same bit for bit.  For captured graphs: a branch of a graph shares the SMs with the other
+// matrices' branches, and a launch that needs several whole SMs at once holds those up.
+static inline size_t chain_ustep_smem(int64_t rb, int64_t vs) { return (size_t)(CH_NB * CH_NB + 2560 + 3 * CH_NB * rb) * vs; }
+template <typename T, int TR, int RB>
+__global__ void __launch_bounds__(CH_THREADS) k_chain_ustep(const ChainFront *__restrict__ fr, int K, int nb, int64_t f0, int64_t U0,
+                                                            int np_last, const T *__restrict__ Ua, const T *__restrict__ pk, T *Y, T *X,
+                                                            int64_t n, int rb, int s, T *gacc, const DevStatus *st)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int tid = threadIdx.x, o = quad_o(tid), q = quad_q(tid), t = s + 1 + blockIdx.x;
+    T *M = reinterpret_cast<T *>(smem_raw), *tr = M + CH_NB * CH_NB, *xp = tr + 2560, *ys = xp + CH_NB * RB, *x = ys + CH_NB * RB;
+    auto front_of = [&](int u) -> int { return TR == 0 ? K - 1 - u : u; };
+    auto np_of = [&](int u) -> int { return front_of(u) == K - 1 ? np_last : nb; };
+    auto f_of = [&](int u) -> int64_t { return f0 + (int64_t)front_of(u) * nb; };
+    auto stage = [&](T *dst, const T *src, int cnt) {
+        for (int e0 = tid; e0 < cnt; e0 += 16 * CH_THREADS) {
+            T v[16];
+#pragma unroll
+            for (int z = 0; z < 16; z++) v[z] = e0 + z * CH_THREADS < cnt ? src[e0 + z * CH_THREADS] : VT<T>::zero();
+#pragma unroll
+            for (int z = 0; z < 16; z++) if (e0 + z * CH_THREADS < cnt) dst[e0 + z * CH_THREADS] = v[z];
+        }
+    };
+    const int np = np_of(t);
+    if (s >= 0) {                                      // (the factors do not change during the solve: before the wait)
+        const int a = TR == 0 ? front_of(t) : front_of(s), c = TR == 0 ? front_of(s) : front_of(t);
+        stage(M, Ua + U0 + (int64_t)nb * ((int64_t)a * (n - f0) - (int64_t)nb * a * (a + 1) / 2) + (int64_t)(c - a - 1) * nb * nb,
+              nb * (c == K - 1 ? np_last : nb));
+    }
+    if (blockIdx.x == 0) stage(tr, pk + fr[front_of(t)].u_pk, (int)pk_u((np + 15) >> 4));
+    pdl_wait();
+    pdl_trigger();
+    if (st->code) return;
+    for (int e = tid; e < CH_NB * RB; e += CH_THREADS) {
+        const int k = e & (CH_NB - 1), r = e / CH_NB;
+        xp[k * RB + r] = s >= 0 && r < rb && k < np_of(s) ? ldcg_v(X + f_of(s) + k + r * n) : VT<T>::zero();
+        if (blockIdx.x == 0) {
+            ys[k * RB + r] = r < rb && k < np ? ldcg_v(Y + f_of(t) + k + r * n) : VT<T>::zero();
+            x[k * RB + r] = VT<T>::zero();
+        }
+    }
+    __syncthreads();
+    T a[RB];
+    if (s >= 0) {
+        const int no = TR == 0 ? (blockIdx.x == 0 ? np : nb) : np, kn = blockIdx.x == 0 ? np_of(s) : TR == 0 ? np_of(s) : nb;
+        block_mv<T, TR, RB>(a, M, nb, o < no ? o : 0, q, kn, xp);
+        if (q == 0 && o < no) {
+            if (blockIdx.x == 0) {
+#pragma unroll
+                for (int r = 0; r < RB; r++) ys[o * RB + r] = sub(ys[o * RB + r], a[r]);
+            } else {
+                T *ao = gacc + ((int64_t)t * CH_NB + o) * RB;
+#pragma unroll
+                for (int r = 0; r < RB; r++) a[r] = add(s > 0 ? ao[r] : VT<T>::zero(), a[r]);
+                if (s == t - 2) {
+#pragma unroll
+                    for (int r = 0; r < RB; r++) if (r < rb) { T *y = Y + f_of(t) + o + r * n; *y = sub(*y, a[r]); }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < RB; r++) ao[r] = a[r];
+                }
+            }
+        }
+    }
+    if (blockIdx.x > 0) return;
+    __syncthreads();
+    chain_tri<T, TR, RB>(tr, ys, x, (np + 15) >> 4, o, q);
+    __syncthreads();
+    for (int e = tid; e < np * rb; e += CH_THREADS) { const int k = e % np, r = e / np; X[f_of(t) + k + r * n] = x[k * RB + r]; }
+}
+
+// dynamic shared memory of k_chain_l: CH_LSTAGES packed pieces, two row vectors
 constexpr int CH_LSTAGES = 4;
+__host__ __device__ constexpr int ch_lpiece(int maxnr) { return 256 + 16 * maxnr; }
 static inline size_t chain_l_smem(int64_t maxnr, int64_t rb, int64_t vs)
 {
-    return (size_t)(CH_LSTAGES * (16 * maxnr + 256) + 2 * maxnr * rb) * vs;
+    return (size_t)(CH_LSTAGES * ch_lpiece((int)maxnr) + 2 * (maxnr + 16) * rb) * vs;
 }
 
 // The L sweep (TR 0: v0 = the first front's gathered vector in its final row order, VB; later fronts' entering rows from R
 // in row space; y into S2 in pivot order) or the L^T sweep (TR 1, 2: z = R in pivot order; x into S2).  blockIdx.x: the
 // group of RB right-hand sides.
 template <typename T, int TR, int RB>
-__global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__restrict__ fr, int K, int maxnr, const T *__restrict__ La,
-                                                        const T *__restrict__ dinv, const int *__restrict__ permall,
-                                                        const int64_t *__restrict__ rowinit, const T *__restrict__ VB0, int64_t vstride,
-                                                        const T *__restrict__ R, T *__restrict__ S2, int64_t n, int nrhs)
+__global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__restrict__ fr, int K, int maxnr, const T *__restrict__ pk,
+                                                        const int *__restrict__ permall, const int64_t *__restrict__ rowinit,
+                                                        const T *__restrict__ VB0, int64_t vstride, const T *__restrict__ R,
+                                                        T *__restrict__ S2, int64_t n, int nrhs, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ unsigned long long bars[CH_LSTAGES];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x;
     const int r0 = blockIdx.x * RB, rb = nrhs - r0 < RB ? nrhs - r0 : RB;
-    const int psz = 16 * maxnr + 256;
-    T *ring = reinterpret_cast<T *>(smem_raw);         // piece: L[row, 16b + c] at c * maxnr + row, then the inverted diagonal block
-    T *v = ring + CH_LSTAGES * psz, *vn = v + maxnr * rb;      // the front's row vector: v[pos + r * maxnr]
+    const int psz = ch_lpiece(maxnr), vld = maxnr + 16;
+    T *ring = reinterpret_cast<T *>(smem_raw);
+    T *v = ring + CH_LSTAGES * psz, *vn = v + vld * RB;        // the front's row vector: v[pos * RB + r]
     R += (int64_t)r0 * n; S2 += (int64_t)r0 * n; VB0 += (int64_t)r0 * vstride;
-    // the pieces in order: TR 0: fronts and blocks ascending, else descending
-    int pk = TR == 0 ? 0 : K - 1, pb = TR == 0 ? 0 : ((int)fr[K - 1].np + 15) / 16 - 1;
-    auto load_next = [&](int slot) {
-        if (pk >= 0 && pk < K) {
-            const ChainFront F = fr[pk];
-            const int np = (int)F.np, nr = (int)F.nr, k0 = 16 * pb, w = np - k0 < 16 ? np - k0 : 16;
-            T *d = ring + slot * psz;
-            for (int c = warp; c < w; c += CH_THREADS / 32)
-                for (int row = k0 + 16 + lane; row < nr; row += 32) cp_async_el(d + c * maxnr + row, La + F.L_off + row + (int64_t)(k0 + c) * F.nr);
-            // (a last block of fewer than 16 pivots: the rows from its end on)
-            if (w < 16) for (int c = warp; c < w; c += CH_THREADS / 32)
-                for (int row = k0 + w + lane; row < nr && row < k0 + 16; row += 32) cp_async_el(d + c * maxnr + row, La + F.L_off + row + (int64_t)(k0 + c) * F.nr);
-            cp_async_el(d + 16 * maxnr + tid, dinv + ((int64_t)pk * 8 + 4 + pb) * 256 + tid);
-            if (TR == 0) { if (k0 + 16 < np) pb++; else { pk++; pb = 0; } }
-            else { if (pb > 0) pb--; else { pk--; if (pk >= 0) pb = ((int)fr[pk].np + 15) / 16 - 1; } }
-        }
-        cp_async_commit();
-    };
-    for (int k = 0; k < CH_LSTAGES - 1; k++) load_next(k);
-    int slot = 0;
-    if (TR == 0) {
-        for (int e = tid; e < (int)fr[0].nr * rb; e += CH_THREADS) { const int p = e % (int)fr[0].nr, r = e / (int)fr[0].nr; v[p + r * maxnr] = VB0[p + r * vstride]; }
-    } else {
-        const ChainFront F = fr[K - 1];
-        for (int e = tid; e < (int)F.np * rb; e += CH_THREADS) { const int p = e % (int)F.np, r = e / (int)F.np; v[p + r * maxnr] = R[F.f + p + r * n]; }
+    if (tid == 0) {
+        s_ok = st->code == 0;
+        for (int k = 0; k < CH_LSTAGES; k++) bar_init(bars + k, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int e = tid; e < 2 * vld * RB; e += CH_THREADS) v[e] = VT<T>::zero();
+    __syncthreads();
+    if (!*(volatile int *)&s_ok) return;
+    // the pieces in order: TR 0: fronts and blocks ascending, else descending (the loading thread; the front after the
+    // one being loaded is read ahead)
+    const bool loader = tid == CH_THREADS - 1;
+    const int step = TR == 0 ? 1 : -1;
+    int pkf = TR == 0 ? 0 : K - 1, issued = 0;
+    ChainFront PF = fr[pkf], PN = fr[K > 1 ? pkf + step : pkf];
+    int pb = TR == 0 ? 0 : ((int)PF.np + 15) / 16 - 1;
+    auto load_next = [&]() {
+        if (pkf < 0 || pkf >= K) return;
+        const int np = (int)PF.np, k0 = 16 * pb, w = np - k0 < 16 ? np - k0 : 16;
+        const unsigned bytes = (unsigned)((256 + 16 * ((int)PF.nr - k0 - w)) * sizeof(T));
+        unsigned long long *bar = bars + issued % CH_LSTAGES;
+        bulk_expect(bar, bytes);
+        bulk_load(ring + (issued % CH_LSTAGES) * psz, pk + PF.l_pk + pk_l(pb, PF.nr), bytes, bar);
+        issued++;
+        const bool end = TR == 0 ? k0 + 16 >= np : pb == 0;
+        if (!end) { pb += step; return; }
+        pkf += step;
+        PF = PN;
+        pb = TR == 0 ? 0 : ((int)PF.np + 15) / 16 - 1;
+        if (pkf + step >= 0 && pkf + step < K) PN = fr[pkf + step];
+    };
+    if (loader) for (int k = 0; k < CH_LSTAGES - 1; k++) load_next();
+    ChainFront F = fr[TR == 0 ? 0 : K - 1];
+    {
+        const int m = TR == 0 ? (int)F.nr : (int)F.np;
+        for (int e = tid; e < m * rb; e += CH_THREADS) { const int p = e % m, r = e / m; v[p * RB + r] = TR == 0 ? VB0[p + r * vstride] : R[F.f + p + r * n]; }
+    }
+    int done = 0;
     for (int kk = 0; kk < K; kk++) {
         const int k = TR == 0 ? kk : K - 1 - kk;
-        const ChainFront F = fr[k];
         const int np = (int)F.np, nr = (int)F.nr, nbk = (np + 15) >> 4;
-        // for the next front: this thread's row position there (TR 0), or here (TR 1, 2: where it came from)
-        int pm = -1;
+        const bool more = kk + 1 < K;
+        const ChainFront N = fr[more ? k + step : k];  // the next front
+        // G: the front whose rows enter from the one below it (the next one, TR 0; this one otherwise); this thread's row there
+        const int gnr = TR == 0 ? (int)N.nr : nr, gsl = (int)(TR == 0 ? N.slot : F.slot), gns = (int)(TR == 0 ? N.nslot : F.nslot),
+                  gta = (int)(TR == 0 ? N.tau : F.tau);
+        const int64_t gro = TR == 0 ? N.row_off : F.row_off;
+        int pm = more && tid < gnr ? permall[gro + tid] : -1, t = -1;
+        int64_t g = -1;
         T ent[RB];
-        const int kn = TR == 0 ? k + 1 : k - 1;        // the next front
-        const ChainFront G = TR == 0 ? fr[kn < K ? kn : k] : F;        // the front whose rows enter from the one below it
-        const bool more = TR == 0 ? kn < K : kn >= 0;
-        if (more && tid < (int)G.nr) pm = permall[G.row_off + tid];
-        for (int bb = 0; bb < nbk; bb++) {
-            const int b = TR == 0 ? bb : nbk - 1 - bb, k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16;
-            cp_async_wait_n<CH_LSTAGES - 2>();
-            __syncthreads();
-            load_next((slot + CH_LSTAGES - 1) % CH_LSTAGES);
-            const T *Lp = ring + slot * psz, *D = Lp + 16 * maxnr;
-            slot = (slot + 1) % CH_LSTAGES;
+#pragma unroll
+        for (int r = 0; r < RB; r++) ent[r] = VT<T>::zero();
+        if (TR != 0 && more && tid < (int)N.np)
+#pragma unroll
+            for (int r = 0; r < RB; r++) if (r < rb) ent[r] = R[N.f + tid + r * n];
+        for (int bb = 0; bb < nbk; bb++, done++) {
+            const int b = TR == 0 ? bb : nbk - 1 - bb, k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16, rl = nr - k0 - w;
+            if (!bar_wait(bars + done % CH_LSTAGES, (unsigned)(done / CH_LSTAGES) & 1u)) s_ok = 0;
+            __syncthreads();                           // (the piece before is no longer read: its stage is the next to load)
+            if (!*(volatile int *)&s_ok) {
+                if (tid == 0) set_status(st, ST_WAIT, k, 0, 0);
+                if (loader) for (; done < issued; done++) (void)bar_wait(bars + done % CH_LSTAGES, (unsigned)(done / CH_LSTAGES) & 1u);
+                return;
+            }
+            const T *D = ring + (done % CH_LSTAGES) * psz, *Lp = D + 256;      // Lp[c * rl + (row - k0 - w)]
             T a[RB];
             if (TR == 0) {
                 if (tid < 64) {
-                    const int o = tid >> 2, q = tid & 3;
-                    quad_mv<T, 0, RB>(a, D, 16, o, q, w, v + k0, maxnr, rb);
-                    __syncwarp();
-                }
-                __syncthreads();
-                if (tid < 64 && (tid & 3) == 0 && (tid >> 2) < w) {
-                    const int o = tid >> 2;
+                    quad_mv<T, 0, RB>(a, D, 16, quad_o(tid), quad_q(tid), 16, v + k0 * RB);   // (past the pivots: zero columns of the inverse's rows)
+                    named_bar(2, 64);
+                    if (quad_q(tid) == 0 && quad_o(tid) < w) {
+                        const int oo = quad_o(tid);
 #pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rb) { v[k0 + o + r * maxnr] = a[r]; S2[F.f + k0 + o + r * n] = a[r]; }
+                        for (int r = 0; r < RB; r++) { v[(k0 + oo) * RB + r] = a[r]; if (r < rb) S2[F.f + k0 + oo + r * n] = a[r]; }
+                    }
+                } else if (loader) load_next();
+                // the next front's rows, a block step after the load each needs (so that none waits)
+                if (bb == (nbk > 1 ? 1 : 0) && pm >= 0) {
+                    t = pm >= gsl && pm < gsl + gns ? pm - gsl : pm >= gta ? gns + pm - gta : -1;
+                    if (t < 0) g = rowinit[gro + pm];
                 }
+                if (bb == nbk - 1 && pm >= 0 && t < 0 && g >= 0)
+#pragma unroll
+                    for (int r = 0; r < RB; r++) if (r < rb) ent[r] = R[g + r * n];
                 __syncthreads();
                 // the rows below: two lanes per row, eight columns each
-                for (int i0 = k0 + w; i0 < nr; i0 += CH_THREADS / 2) {
-                    const int row = i0 + (tid >> 1), h = tid & 1;
+                for (int i0 = 0; i0 < rl; i0 += CH_THREADS / 2) {
+                    const int i = i0 + (tid & 15) + 16 * (tid >> 5), h = (tid >> 4) & 1, ii = i < rl ? i : 0;
                     T s[RB];
 #pragma unroll
                     for (int r = 0; r < RB; r++) s[r] = VT<T>::zero();
-                    if (row < nr) {
 #pragma unroll
-                        for (int c = 0; c < 8; c++) {
-                            const int cc = 2 * c + h;
-                            if (cc < w) {
-                                const T l = Lp[cc * maxnr + row];
+                    for (int c = 0; c < 8; c++) {
+                        const T l = Lp[(2 * c + h) * rl + ii];
+                        const T *xv = v + (k0 + (2 * c + h < w ? 2 * c + h : 0)) * RB;
 #pragma unroll
-                                for (int r = 0; r < RB; r++) if (r < rb) s[r] = madd<T>(s[r], l, v[k0 + cc + r * maxnr]);
-                            }
-                        }
+                        for (int r = 0; r < RB; r++) s[r] = madd<T>(s[r], l, xv[r]);
                     }
 #pragma unroll
                     for (int r = 0; r < RB; r++) {
-                        s[r] = add(s[r], shfl_xor_v<T>(s[r], 1));
-                        if (r < rb && row < nr && h == 0) v[row + r * maxnr] = sub(v[row + r * maxnr], s[r]);
+                        s[r] = add(s[r], shfl_xor_v<T>(s[r], 16));
+                        if (i < rl && h == 0) v[(k0 + w + i) * RB + r] = sub(v[(k0 + w + i) * RB + r], s[r]);
                     }
                 }
             } else {
+                if (loader) load_next();
+                if (bb == (nbk > 1 ? 1 : 0) && pm >= 0) t = pm >= gsl && pm < gsl + gns ? pm - gsl : pm >= gta ? gns + pm - gta : -1;
                 // s_b = z_b - L[rows below, b]^T x: sixteen lanes per column
                 const int c = tid >> 4, l16 = tid & 15;
                 T s[RB];
 #pragma unroll
                 for (int r = 0; r < RB; r++) s[r] = VT<T>::zero();
-                if (c < w)
-                    for (int row = k0 + w + l16; row < nr; row += 16) {
-                        const T l = opv<TR>(Lp[c * maxnr + row]);
+                for (int i = l16; i < rl; i += 16) {
+                    const T l = opv<TR>(Lp[c * rl + i]);
 #pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rb) s[r] = madd<T>(s[r], l, v[row + r * maxnr]);
-                    }
+                    for (int r = 0; r < RB; r++) s[r] = madd<T>(s[r], l, v[(k0 + w + i) * RB + r]);
+                }
 #pragma unroll
                 for (int r = 0; r < RB; r++) {
 #pragma unroll
                     for (int m = 8; m > 0; m >>= 1) s[r] = add(s[r], shfl_xor_v<T>(s[r], m));
-                    if (r < rb && c < w && l16 == 0) v[k0 + c + r * maxnr] = sub(v[k0 + c + r * maxnr], s[r]);
+                    if (c < w && l16 == 0) v[(k0 + c) * RB + r] = sub(v[(k0 + c) * RB + r], s[r]);
                 }
                 __syncthreads();
-                if (tid < 64) quad_mv<T, TR, RB>(a, D, 16, tid >> 2, tid & 3, w, v + k0, maxnr, rb);
-                __syncthreads();
-                if (tid < 64 && (tid & 3) == 0 && (tid >> 2) < w) {
-                    const int o = tid >> 2;
+                if (tid < 64) {
+                    // (a last block of fewer than 16 pivots: the rows after it are not part of it)
+                    const int oo = quad_o(tid), q = quad_q(tid);
 #pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rb) { v[k0 + o + r * maxnr] = a[r]; S2[F.f + k0 + o + r * n] = a[r]; }
+                    for (int r = 0; r < RB; r++) a[r] = VT<T>::zero();
+#pragma unroll
+                    for (int z = 0; z < 4; z++) {
+                        const int kq = (4 * q + z + oo) & 15;
+                        const T m = opv<TR>(D[oo * 16 + kq]);
+                        if (kq < w)
+#pragma unroll
+                            for (int r = 0; r < RB; r++) a[r] = madd<T>(a[r], m, v[(k0 + kq) * RB + r]);
+                    }
+                    quad_sum<T, RB>(a);
+                    named_bar(2, 64);
+                    if (q == 0 && oo < w)
+#pragma unroll
+                        for (int r = 0; r < RB; r++) { v[(k0 + oo) * RB + r] = a[r]; if (r < rb) S2[F.f + k0 + oo + r * n] = a[r]; }
                 }
             }
         }
         if (!more) break;
         // the next front's vector
-        int t = -1;                                    // the contribution row (of the front below G) at this position of G
-        if (pm >= 0) t = pm >= (int)G.slot && pm < (int)(G.slot + G.nslot) ? pm - (int)G.slot : pm >= (int)G.tau ? (int)G.nslot + pm - (int)G.tau : -1;
+        __syncthreads();
         if (TR == 0) {
-            if (pm >= 0 && t < 0) {
-                const int64_t g = rowinit[G.row_off + pm];
-#pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) ent[r] = g >= 0 ? R[g + r * n] : VT<T>::zero();
-            }
-            __syncthreads();
             if (pm >= 0)
 #pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) vn[tid + r * maxnr] = t >= 0 ? v[np + t + r * maxnr] : ent[r];
+                for (int r = 0; r < RB; r++) vn[tid * RB + r] = t >= 0 ? v[(np + t) * RB + r] : ent[r];
         } else {
-            const ChainFront H = fr[kn];
-            T z[RB];
-            if (tid < (int)H.np)
-#pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) z[r] = R[H.f + tid + r * n];
-            __syncthreads();
             if (t >= 0)
 #pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) vn[(int)H.np + t + r * maxnr] = v[tid + r * maxnr];
-            if (tid < (int)H.np)
+                for (int r = 0; r < RB; r++) vn[((int)N.np + t) * RB + r] = v[tid * RB + r];
+            if (tid < (int)N.np)
 #pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rb) vn[tid + r * maxnr] = z[r];
+                for (int r = 0; r < RB; r++) vn[tid * RB + r] = ent[r];
         }
         T *sw = v; v = vn; vn = sw;
+        F = N;
         // (the next piece's barrier orders these writes before they are read)
     }
-    cp_async_wait_n<0>();
 }
 
 }  // namespace fpl

@@ -326,61 +326,52 @@ __global__ void __launch_bounds__(512) k_panel(T *__restrict__ W, int64_t ld, in
     }
 }
 
-// The partial-pivot LU of a tall front's pivot block (nrows x npiv, too large for one CTA's shared memory) in one launch
-// over G CTAs resident at once: one thread-block cluster (G <= MC_CMAX: the CTAs exchange their candidates through
-// distributed shared memory and the cluster barrier), or a cooperative launch (G up to one CTA per SM: the candidates go
-// through global memory and a counter that every CTA increments).  CTA b owns the rows [b * per, b * per + per) and
+// The partial-pivot LU of the tallest fronts' pivot blocks (nrows x npiv, more rows than one cluster's CTAs take: see
+// block_lu_cl.cuh) in one cooperative launch of up to one CTA per SM.  CTA b owns the rows [b * per, b * per + per) and
 // keeps its rows' values of the current 32-column panel in shared memory.  Per pivot column j:
-//   1. each CTA finds the best of its live rows (the largest pivot key, ties to the smaller row of B) and posts it: the
-//      key, the row of B, the position and the row's panel values (cluster: into every CTA's shared memory; grid: into
-//      its global slot, then a release increment of the counter);
-//   2. after the barrier (the cluster barrier; grid: the counter reaching G (j + 1), a bounded wait) every CTA takes the
-//      same winner, applies the same singular / border decision (a stop ends every CTA at the same column), keeps the
-//      winner's panel values (row j of L11\U11) and updates its live rows: the multiplier, then the rank-1 update of the
-//      panel's later columns.
+//   1. each CTA finds the best of its live rows (the largest pivot key, ties to the smaller row of B) and posts it into its
+//      global slot: the key, the row of B, the position and the row's panel values, then a release increment of the counter;
+//   2. once the counter reaches G (j + 1) (a bounded wait) every CTA takes the same winner, applies the same singular /
+//      border decision (a stop ends every CTA at the same column), keeps the winner's panel values (row j of L11\U11) and
+//      updates its live rows: the multiplier, then the rank-1 update of the panel's later columns.
 // After a panel every CTA forms U12 = L11^-1 A12 for the panel's pivot rows (read from W: their owners wrote them before
 // posting the panel's first column), by column chunks and redundantly, and applies A22 -= L21 U12 to its own live rows;
 // one CTA per chunk keeps U12 in Ub for the final block.  Rows never move: the pivot rows are marked, and k_mc_order /
 // k_mc_lout turn the choices (chosen[j] = the position of step j's pivot row) into the final row order (the pivot rows
 // in step order, then the others in their order) and the block in that order.  The operations on every value are those
 // of the swapping form (the same multipliers, the same forward substitution order), so the factors agree with it.
-// The posts alternate by the column's parity.  Grid form: sync[0] is the exit ticket, sync[1] the counter; the last CTA
-// to finish resets both, so they start at zero at the next launch (a CUDA graph replay included).
-constexpr int MC_THREADS = 512, MC_PW = 32, MC_LB = MC_PW + 1, MC_CMAX = 16;
+// The posts alternate by the column's parity.  sync[0] is the exit ticket, sync[1] the counter; the last CTA to finish
+// resets both, so they start at zero at the next launch (a CUDA graph replay included).
+constexpr int MC_THREADS = 512, MC_PW = 32, MC_LB = MC_PW + 1;
 constexpr unsigned MC_SPIN = 1u << 22;         // polls of the counter before the wait gives up (about a second)
 template <typename T> struct __align__(16) McSlot {
     long long key, rid, pos, pad;
     T v[MC_PW];
 };
 template <typename T> __host__ __device__ constexpr int mc_cw() { return VT<T>::cplx_ ? 64 : 128; }
-// shared memory of k_block_lu_mc for `per` rows per CTA (cl: the cluster form's posts too)
-template <typename T> __host__ __device__ constexpr size_t mc_smem(int per, bool cl)
+// shared memory of k_block_lu_mc for `per` rows per CTA
+template <typename T> __host__ __device__ constexpr size_t mc_smem(int per)
 {
-    return (size_t)(MC_PW * per + MC_PW * MC_LB + MC_PW * mc_cw<T>()) * sizeof(T) +
-           (cl ? (size_t)2 * MC_CMAX * sizeof(McSlot<T>) : 0) + (size_t)per * 8 + (size_t)((per + 15) & ~15);
+    return (size_t)(MC_PW * per + MC_PW * MC_LB + MC_PW * mc_cw<T>()) * sizeof(T) + (size_t)per * 8 + (size_t)((per + 15) & ~15);
 }
 
-template <typename T, bool CL>
+template <typename T>
 __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, int nrows, int npiv, int nri, int per,
                                                           int64_t fcol, const double *__restrict__ colmax, double pivot_rel,
                                                           const int64_t *__restrict__ rowid, int64_t *__restrict__ chosen,
                                                           T *__restrict__ Ub, McSlot<T> *gslots, unsigned int *sync,
                                                           DevStatus *st, int64_t front)
 {
-    namespace cg = cooperative_groups;
     constexpr int CW = mc_cw<T>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *S = reinterpret_cast<T *>(smem_raw);              // the panel: S[c * per + r], own row r, panel column c
     T *Lb = S + MC_PW * per;                             // the panel's pivot rows: Lb[k * MC_LB + c] (L11 \ U11)
     T *Uc = Lb + MC_PW * MC_LB;                          // a chunk of U12: Uc[k * CW + c]
-    McSlot<T> *cs = reinterpret_cast<McSlot<T> *>(Uc + MC_PW * CW);    // cluster form: the posts, [parity][CTA]
-    long long *rid_s = reinterpret_cast<long long *>(reinterpret_cast<unsigned char *>(cs) +
-                                                     (CL ? (size_t)2 * MC_CMAX * sizeof(McSlot<T>) : 0));
+    long long *rid_s = reinterpret_cast<long long *>(Uc + MC_PW * CW);
     unsigned char *live = reinterpret_cast<unsigned char *>(rid_s + per);
     __shared__ long long s_k[16], s_r[16], s_p[16];
     __shared__ int s_q[16];
     __shared__ int s_piv[MC_PW];
-    __shared__ T s_wc[16 * MC_PW];                      // cluster form: each warp's candidate row, fully updated
     __shared__ double s_thr[MC_PW];
     __shared__ int s_stop, s_wait;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = MC_THREADS / 32;
@@ -391,11 +382,6 @@ __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, in
     for (int r = tid; r < per; r += MC_THREADS) {
         live[r] = r < nmine;
         rid_s[r] = r < nmine ? rowid[r_lo + r] : LLONG_MAX;
-    }
-    if constexpr (CL) {
-        // every CTA of the cluster starts from CTA 0's reading of the status word (the barrier counts must agree)
-        cg::this_cluster().sync();
-        if (tid == 0) s_stop = *cg::this_cluster().map_shared_rank(&s_stop, 0);
     }
     __syncthreads();
     bool stopped = s_stop != 0;                          // the same in every thread (every decision below is)
@@ -421,99 +407,65 @@ __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, in
                 brid = src >= 0 ? __shfl_sync(0xffffffffu, brid, src) : LLONG_MAX;
                 brow = src >= 0 ? __shfl_sync(0xffffffffu, brow, src) : -1;
             }
-            if constexpr (CL) {
-                // the warp's candidate row in full: its later columns still lack the previous pivot's update (applied
-                // to every row during the cluster barrier below), so it is applied here, with the same arithmetic
-                __syncwarp();
-                if (lane < w) {
-                    T v = brow >= 0 ? S[lane * per + brow] : VT<T>::zero();
-                    if (brow >= 0 && kk >= 1 && lane > kk)
-                        v = sub(v, mul(S[(kk - 1) * per + brow], Lb[(kk - 1) * MC_LB + lane]));
-                    s_wc[warp * MC_PW + lane] = v;
-                }
-            }
             if (lane == 0) { s_k[warp] = bk; s_r[warp] = brid; s_p[warp] = brow; }
             __syncthreads();
-            if (CL ? warp < G : warp == 0) {
-                // the CTA's best (cluster form: every pushing warp takes it; warp d pushes it into CTA d)
+            if (warp == 0) {
+                // the CTA's best
                 bk = lane < nw ? s_k[lane] : -1; brid = lane < nw ? s_r[lane] : LLONG_MAX; brow = lane < nw ? s_p[lane] : -1;
                 const int src = warp_argbest(bk, brid);
                 bk = src >= 0 ? __shfl_sync(0xffffffffu, bk, src) : -1;
                 brid = src >= 0 ? __shfl_sync(0xffffffffu, brid, src) : LLONG_MAX;
                 brow = src >= 0 ? __shfl_sync(0xffffffffu, brow, src) : -1;
-                const T v = (lane < w && brow >= 0) ? (CL ? s_wc[src * MC_PW + lane] : S[lane * per + brow]) : VT<T>::zero();
+                const T v = (lane < w && brow >= 0) ? S[lane * per + brow] : VT<T>::zero();
                 const long long pos = brow >= 0 ? r_lo + brow : -1;
-                if constexpr (CL) {
-                    McSlot<T> *dst = cg::this_cluster().map_shared_rank(cs + par * MC_CMAX + b, warp);
-                    if (lane < w) dst->v[lane] = v;
-                    if (lane == 0) { dst->key = bk; dst->rid = brid; dst->pos = pos; }
-                } else {
-                    McSlot<T> *my = gslots + (size_t)par * G + b;
-                    if (lane < w) my->v[lane] = v;
-                    if (lane == 0) { my->key = bk; my->rid = brid; my->pos = pos; }
-                    __syncwarp();
-                    if (lane == 0) {
-                        red_release_add_u32(sync + 1, 1u);
-                        const unsigned target = (unsigned)G * (unsigned)(j + 1);
-                        unsigned it = 0;
-                        while (ld_acquire_u32(sync + 1) < target && ++it < MC_SPIN) {}
-                        if (it >= MC_SPIN) s_wait = 1;
-                    }
+                McSlot<T> *my = gslots + (size_t)par * G + b;
+                if (lane < w) my->v[lane] = v;
+                if (lane == 0) { my->key = bk; my->rid = brid; my->pos = pos; }
+                __syncwarp();
+                if (lane == 0) {
+                    red_release_add_u32(sync + 1, 1u);
+                    const unsigned target = (unsigned)G * (unsigned)(j + 1);
+                    unsigned it = 0;
+                    while (ld_acquire_u32(sync + 1) < target && ++it < MC_SPIN) {}
+                    if (it >= MC_SPIN) s_wait = 1;
                 }
             }
             // 2. the barrier, then the same winner in every warp
             long long gk = -1, gr = LLONG_MAX, gp = -1;
             int gq = -1;
             const T *wv;                                 // the winner's panel values
-            if constexpr (CL) {
-                asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-                // while the other CTAs arrive: the previous pivot's update of this row's later columns
-                if (mine && kk >= 1) {
-                    const T l = S[(kk - 1) * per + tid];
-                    for (int c = kk + 1; c < w; c++) S[c * per + tid] = sub(S[c * per + tid], mul(l, Lb[(kk - 1) * MC_LB + c]));
-                }
-                asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-                if (lane < G) {
-                    const McSlot<T> *c = cs + par * MC_CMAX + lane;
-                    gk = c->key; gr = c->rid; gp = c->pos; gq = lane;
-                }
-                const int src = warp_argbest(gk, gr);
-                gp = src >= 0 ? __shfl_sync(0xffffffffu, gp, src) : -1;
-                gq = src >= 0 ? __shfl_sync(0xffffffffu, gq, src) : -1;
-                gk = src >= 0 ? __shfl_sync(0xffffffffu, gk, src) : -1;
-                wv = gq >= 0 ? cs[par * MC_CMAX + gq].v : Lb + kk * MC_LB;
-            } else {
-                __syncthreads();
-                if (tid < G && !s_wait) {
-                    const McSlot<T> *c = gslots + (size_t)par * G + tid;
-                    gk = __ldcg(&c->key); gr = __ldcg(&c->rid); gp = __ldcg(&c->pos); gq = tid;
-                }
-                {
-                    const int src = warp_argbest(gk, gr);
-                    gk = src >= 0 ? __shfl_sync(0xffffffffu, gk, src) : -1;
-                    gr = src >= 0 ? __shfl_sync(0xffffffffu, gr, src) : LLONG_MAX;
-                    gp = src >= 0 ? __shfl_sync(0xffffffffu, gp, src) : -1;
-                    gq = src >= 0 ? __shfl_sync(0xffffffffu, gq, src) : -1;
-                }
-                if (lane == 0) { s_k[warp] = gk; s_r[warp] = gr; s_p[warp] = gp; s_q[warp] = gq; }
-                __syncthreads();
-                gk = lane < nw ? s_k[lane] : -1; gr = lane < nw ? s_r[lane] : LLONG_MAX;
-                gp = lane < nw ? s_p[lane] : -1; gq = lane < nw ? s_q[lane] : -1;
-                const int src = warp_argbest(gk, gr);
-                gp = src >= 0 ? __shfl_sync(0xffffffffu, gp, src) : -1;
-                gq = src >= 0 ? __shfl_sync(0xffffffffu, gq, src) : -1;
-                gk = src >= 0 ? __shfl_sync(0xffffffffu, gk, src) : -1;
-                // warp 0 brings the winner's values into Lb for every warp
-                if (warp == 0 && lane < w)
-                    Lb[kk * MC_LB + lane] = gq >= 0 ? ldcg_v(&gslots[(size_t)par * G + gq].v[lane]) : VT<T>::zero();
-                __syncthreads();
-                wv = Lb + kk * MC_LB;
+            __syncthreads();
+            if (tid < G && !s_wait) {
+                const McSlot<T> *c = gslots + (size_t)par * G + tid;
+                gk = __ldcg(&c->key); gr = __ldcg(&c->rid); gp = __ldcg(&c->pos); gq = tid;
             }
+            {
+                const int src = warp_argbest(gk, gr);
+                gk = src >= 0 ? __shfl_sync(0xffffffffu, gk, src) : -1;
+                gr = src >= 0 ? __shfl_sync(0xffffffffu, gr, src) : LLONG_MAX;
+                gp = src >= 0 ? __shfl_sync(0xffffffffu, gp, src) : -1;
+                gq = src >= 0 ? __shfl_sync(0xffffffffu, gq, src) : -1;
+            }
+            if (lane == 0) { s_k[warp] = gk; s_r[warp] = gr; s_p[warp] = gp; s_q[warp] = gq; }
+            __syncthreads();
+            gk = lane < nw ? s_k[lane] : -1; gr = lane < nw ? s_r[lane] : LLONG_MAX;
+            gp = lane < nw ? s_p[lane] : -1; gq = lane < nw ? s_q[lane] : -1;
+            {
+                const int src = warp_argbest(gk, gr);
+                gp = src >= 0 ? __shfl_sync(0xffffffffu, gp, src) : -1;
+                gq = src >= 0 ? __shfl_sync(0xffffffffu, gq, src) : -1;
+                gk = src >= 0 ? __shfl_sync(0xffffffffu, gk, src) : -1;
+            }
+            // warp 0 brings the winner's values into Lb for every warp
+            if (warp == 0 && lane < w)
+                Lb[kk * MC_LB + lane] = gq >= 0 ? ldcg_v(&gslots[(size_t)par * G + gq].v[lane]) : VT<T>::zero();
+            __syncthreads();
+            wv = Lb + kk * MC_LB;
             const T pv = gq >= 0 ? wv[kk] : VT<T>::zero();
             // the decision, the same in every thread
             const double t = s_thr[kk];
             int stop = 0;
-            if (!CL && s_wait) stop = 2;
+            if (s_wait) stop = 2;
             else if (gp < 0 || gk <= 0 || ((unsigned long long)gk < pivkey_of_modulus<T>(2.0 * t) && vabs(pv) < t)) stop = 1;
             else if (gp >= nri) stop = 3;
             if (tid == 0) {
@@ -523,10 +475,6 @@ __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, in
                 if (!stop) { if (b == 0) chosen[j] = gp; s_piv[kk] = (int)gp; }
             }
             if (stop) { stopped = true; break; }
-            if constexpr (CL) {             // every warp keeps the winner's row (the same values) for its deferred update
-                if (lane < w) Lb[kk * MC_LB + lane] = wv[lane];
-                __syncwarp();
-            }
             // 3. this thread's row: the pivot row leaves the search; a live row takes its multiplier and the update of
             // the panel's later columns
             if (mine) {
@@ -535,12 +483,8 @@ __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, in
                     const T inv = recip(pv);
                     const T l = mul(S[kk * per + tid], inv);
                     S[kk * per + tid] = l;
-                    if constexpr (CL) {         // the next column now; the others during the next column's barrier
-                        if (kk + 1 < w) S[(kk + 1) * per + tid] = sub(S[(kk + 1) * per + tid], mul(l, wv[kk + 1]));
-                    } else {
 #pragma unroll 4
-                        for (int c = kk + 1; c < w; c++) S[c * per + tid] = sub(S[c * per + tid], mul(l, wv[c]));
-                    }
+                    for (int c = kk + 1; c < w; c++) S[c * per + tid] = sub(S[c * per + tid], mul(l, wv[c]));
                 }
             }
         }
@@ -629,9 +573,7 @@ __global__ void __launch_bounds__(MC_THREADS) k_block_lu_mc(T *W, int64_t ld, in
         }
     }
     __syncthreads();
-    if constexpr (CL) {
-        cg::this_cluster().sync();            // no CTA leaves while another may still write its shared memory
-    } else if (tid == 0) {
+    if (tid == 0) {
         __threadfence();
         if (atomicAdd(sync, 1u) == (unsigned)(G - 1)) {   // the last CTA out resets the counter and the ticket
             sync[1] = 0u;
@@ -3143,61 +3085,7 @@ __global__ void k_vupdate(const T *__restrict__ V, int64_t n, int nv, const T *_
 // the children's order, the children's contribution entries that land on it (the lists rsp/rsi over the plan's rows,
 // csp/csi over its columns).
 constexpr int SV_RC = 8;              // right-hand sides per pass of the one-CTA sweep kernels
-constexpr int SVB_RC = 16;            // right-hand sides per pass over a larger front's L21 or U12
 constexpr int SV_THREADS = 256;
-
-// L sweep (trans 0) of a level's small fronts, a CTA each: the front's vector in its final row order (position k holds
-// initial row perm[k]: the entering row's right-hand side, then the children's entries that land on it), x = L11^-1 v
-// (the pivot rows, into Y in pivot order), then the contribution u = v[np:] - L21 x into VB
-template <typename T>
-__global__ void __launch_bounds__(SV_THREADS) k_sv_fwdL(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                        const T *__restrict__ La, const int64_t *__restrict__ rowinit,
-                                                        const int *__restrict__ permall, const int64_t *__restrict__ rsp,
-                                                        const int64_t *__restrict__ rsi, const T *__restrict__ R,
-                                                        T *__restrict__ Y, T *__restrict__ VB, int64_t vstride, int64_t n,
-                                                        int nrhs)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const SvFront F = fr[list[blockIdx.x]];
-    const int nr = (int)F.nr, np = (int)(F.np < F.nr ? F.np : F.nr), nri = (int)F.nri, tid = threadIdx.x;
-    T *v = reinterpret_cast<T *>(smem_raw);          // nr x SV_RC (ld nr)
-    T *x = v + nr * SV_RC;                           // np x SV_RC (ld np)
-    T *sT = x + np * SV_RC;                          // 64 x np
-    const T *L = La + F.L_off;
-    const int *perm = permall + F.row_off;
-    pdl_wait();
-    pdl_trigger();
-    for (int r0 = 0; r0 < nrhs; r0 += SV_RC) {
-        const int rc = nrhs - r0 < SV_RC ? nrhs - r0 : SV_RC;
-        for (int e = tid; e < nr * rc; e += SV_THREADS) {
-            const int k = e % nr, r = e / nr, i = F.np > 0 ? perm[k] : k;     // (a front without pivots keeps its order)
-            const int64_t g = F.row_off + i, ri = rowinit[g];
-            T val = (i < nri && ri >= 0) ? R[ri + (int64_t)(r0 + r) * n] : VT<T>::zero();
-            for (int64_t q = rsp[g]; q < rsp[g + 1]; q++) val = add(val, VB[rsi[q] + (int64_t)(r0 + r) * vstride]);
-            v[k + r * nr] = val;
-        }
-        __syncthreads();
-        for (int e = tid; e < np * rc; e += SV_THREADS) x[e] = v[e % np + (e / np) * nr];
-        __syncthreads();
-        blk_trisolve<T, false>(L, nr, np, x, rc, sT, nullptr, nullptr, 0);
-        for (int e = tid; e < np * rc; e += SV_THREADS) Y[F.f + e % np + (int64_t)(r0 + e / np) * n] = x[e];
-        const int m = nr - np;
-        for (int e = tid; e < m * rc; e += SV_THREADS) {
-            const int t = e % m, r = e / m;
-            T acc = VT<T>::zero();
-            for (int k0 = 0; k0 < np; k0 += 8) {
-                T lv[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) lv[q] = k0 + q < np ? L[np + t + (int64_t)(k0 + q) * nr] : VT<T>::zero();
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (k0 + q < np) acc = add(acc, mul(lv[q], x[k0 + q + r * np]));
-            }
-            VB[F.row_off + np + t + (int64_t)(r0 + r) * vstride] = sub(v[np + t + r * nr], acc);
-        }
-        __syncthreads();
-    }
-}
 
 // a larger front's vector (the L sweep), in its final row order, into its own entries of VB
 template <typename T>
@@ -3243,43 +3131,6 @@ __global__ void k_sv_put(const T *__restrict__ Vf, int64_t vstride, int64_t np, 
 {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < np * nrhs; e += (int64_t)gridDim.x * blockDim.x)
         Y[f + e % np + (e / np) * n] = Vf[e % np + (e / np) * vstride];
-}
-
-// U sweep (trans 0) of a level's small fronts, a CTA each: x = U11^-1 (y - U12 x[CB columns]) (the CB columns' x from
-// the fronts above, already solved)
-template <typename T>
-__global__ void __launch_bounds__(SV_THREADS) k_sv_bwdU(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                        const T *__restrict__ La, const T *__restrict__ Ua,
-                                                        const int64_t *__restrict__ cols, const T *__restrict__ Y,
-                                                        T *__restrict__ X, int64_t n, int nrhs, DevStatus *st)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_zero;
-    const SvFront F = fr[list[blockIdx.x]];
-    const int np = (int)F.np, ncb = (int)(F.nc - F.np), tid = threadIdx.x;
-    T *x = reinterpret_cast<T *>(smem_raw);          // np x SV_RC
-    T *sT = x + np * SV_RC;                          // 64 x np
-    T *dinv = sT + 64 * np;                          // 64
-    const T *U12 = Ua + F.U_off;
-    const int64_t *cb = cols + F.col_off + np;
-    pdl_wait();
-    pdl_trigger();
-    for (int r0 = 0; r0 < nrhs; r0 += SV_RC) {
-        const int rc = nrhs - r0 < SV_RC ? nrhs - r0 : SV_RC;
-        for (int e = tid; e < np * rc; e += SV_THREADS) {
-            const int i = e % np, r = e / np;
-            const T *xr = X + (int64_t)(r0 + r) * n;
-            T acc = VT<T>::zero();
-            for (int t = 0; t < ncb; t++) acc = add(acc, mul(U12[i + (int64_t)t * np], xr[cb[t]]));
-            x[e] = sub(Y[F.f + i + (int64_t)(r0 + r) * n], acc);
-        }
-        if (tid == 0) s_zero = 0;
-        __syncthreads();
-        blk_trisolve<T, true>(La + F.L_off, F.nr, np, x, rc, sT, dinv, st, F.f, &s_zero);
-        if (s_zero) return;
-        for (int e = tid; e < np * rc; e += SV_THREADS) X[F.f + e % np + (int64_t)(r0 + e / np) * n] = x[e];
-        __syncthreads();
-    }
 }
 
 // U^T sweep (trans 1; 2 with conj) of a level's small fronts (npiv <= 64), a CTA each: the front's column vector (the
@@ -3486,97 +3337,6 @@ __global__ void __launch_bounds__(256) k_svb_L11(const SvFront *__restrict__ fr,
             const int64_t r = r0 + e / np;
             VB[F.row_off + k + r * vstride] = x[e];
             Y[F.f + k + r * n] = x[e];
-        }
-        __syncthreads();
-    }
-}
-
-// L sweep, 3: u = v[np:] - L21 x on 256 rows per CTA (x from VB), rc2 right-hand sides per pass over L
-template <typename T>
-__global__ void __launch_bounds__(256) k_svb_L21(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                 const T *__restrict__ La, T *__restrict__ VB, int64_t vstride, int nrhs, int rc2)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const SvFront F = fr[list[blockIdx.y]];
-    const int np = (int)(F.np < F.nr ? F.np : F.nr), tid = threadIdx.x;
-    const int64_t rows = F.nr - np, row0 = (int64_t)blockIdx.x * 256;
-    if (np == 0 || row0 >= rows) return;
-    T *xs = reinterpret_cast<T *>(smem_raw);         // np x rc2
-    const T *L = La + F.L_off;
-    const int64_t rr = np + row0 + tid;
-    for (int r0 = 0; r0 < nrhs; r0 += rc2) {
-        const int rc = nrhs - r0 < rc2 ? nrhs - r0 : rc2;
-        for (int e = tid; e < np * rc; e += blockDim.x) xs[e] = VB[F.row_off + e % np + (int64_t)(r0 + e / np) * vstride];
-        __syncthreads();
-        if (rr < F.nr) {
-            T acc[SVB_RC];
-#pragma unroll
-            for (int r = 0; r < SVB_RC; r++) acc[r] = VT<T>::zero();
-            for (int k0 = 0; k0 < np; k0 += 8) {
-                T lv[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) lv[q] = k0 + q < np ? L[rr + (int64_t)(k0 + q) * F.nr] : VT<T>::zero();
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (k0 + q < np)
-#pragma unroll
-                        for (int r = 0; r < SVB_RC; r++)
-                            if (r < rc) acc[r] = add(acc[r], mul(lv[q], xs[k0 + q + r * np]));
-            }
-#pragma unroll
-            for (int r = 0; r < SVB_RC; r++)
-                if (r < rc) {
-                    T *o = VB + F.row_off + rr + (int64_t)(r0 + r) * vstride;
-                    *o = sub(*o, acc[r]);
-                }
-        }
-        __syncthreads();
-    }
-}
-
-// U sweep, 1: the partial products U12 x[CB columns] of chunk blockIdx.x of a front's CB columns (F.nch chunks), a
-// thread per row of U12, into part (the front's partial sums start at F.poff * nrhs); the chunk's x values staged in
-// shared memory, SVB_RC right-hand sides per pass over U12
-template <typename T>
-__global__ void __launch_bounds__(256) k_svb_u12(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                 const T *__restrict__ Ua, const int64_t *__restrict__ cols,
-                                                 const T *__restrict__ X, int64_t n, int nrhs, T *__restrict__ part)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *Xs = reinterpret_cast<T *>(smem_raw);         // chunk x SVB_RC: Xs[k * SVB_RC + r]
-    const SvFront F = fr[list[blockIdx.y]];
-    if (blockIdx.x >= F.nch || F.np == 0) return;
-    const int64_t np = F.np, ncb = F.nc - F.np, chunk = (ncb + F.nch - 1) / F.nch;
-    const int64_t c0 = blockIdx.x * chunk, c1 = c0 + chunk < ncb ? c0 + chunk : ncb;
-    const int cc = (int)(c1 - c0);
-    const T *U12 = Ua + F.U_off;
-    const int64_t *cb = cols + F.col_off + np;
-    T *pp = part + F.poff * nrhs + (int64_t)blockIdx.x * np * nrhs;
-    for (int r0 = 0; r0 < nrhs; r0 += SVB_RC) {
-        const int rc = nrhs - r0 < SVB_RC ? nrhs - r0 : SVB_RC;
-        for (int e = threadIdx.x; e < cc * rc; e += blockDim.x) {
-            const int k = e / rc, r = e - k * rc;
-            Xs[k * SVB_RC + r] = X[cb[c0 + k] + (int64_t)(r0 + r) * n];
-        }
-        __syncthreads();
-        for (int64_t i = threadIdx.x; i < np; i += blockDim.x) {
-            T acc[SVB_RC];
-#pragma unroll
-            for (int r = 0; r < SVB_RC; r++) acc[r] = VT<T>::zero();
-            for (int k0 = 0; k0 < cc; k0 += 8) {
-                T uv[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) uv[q] = k0 + q < cc ? U12[i + (c0 + k0 + q) * np] : VT<T>::zero();
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (k0 + q < cc)
-#pragma unroll
-                        for (int r = 0; r < SVB_RC; r++)
-                            if (r < rc) acc[r] = add(acc[r], mul(uv[q], Xs[(k0 + q) * SVB_RC + r]));
-            }
-#pragma unroll
-            for (int r = 0; r < SVB_RC; r++)
-                if (r < rc) pp[i + (int64_t)(r0 + r) * np] = acc[r];
         }
         __syncthreads();
     }

@@ -3,6 +3,9 @@
 #include "numeric.hpp"
 #include "kernels.cuh"
 #include "front_lu.cuh"
+#include "block_lu_cl.cuh"
+#include "chain_solve.cuh"
+#include "sweeps.cuh"
 #include "schur_tc.hpp"
 #include <algorithm>
 #include <cstring>
@@ -89,7 +92,7 @@ DevPlan::~DevPlan()
 {
     for (void *p : {(void *)cols, (void *)relcol, (void *)rowinit, (void *)asm_src, (void *)asm_dst, (void *)Bp, (void *)Bi,
                     (void *)Bsrc, (void *)row_perm, (void *)col_perm, (void *)seg, (void *)chain_uoff, (void *)sv, (void *)sv_rows, (void *)sv_cols, (void *)rsp, (void *)rsi, (void *)csp,
-                    (void *)csi, (void *)iota, (void *)sv_brows, (void *)sv_bcols, (void *)fc, (void *)children, (void *)bs_list})
+                    (void *)csi, (void *)iota, (void *)sv_brows, (void *)sv_bcols, (void *)fc, (void *)children, (void *)bs_list, (void *)ch_fronts, (void *)dfront})
         if (p) cudaFree(p);
 }
 
@@ -110,18 +113,34 @@ static int upload_segments(int64_t n, const std::vector<int64_t> &Bp, DevPlan &D
 // (U, U^T) likewise with its columns and U12; the dense chain's fronts, which the U sweep takes by its own kernels, go
 // with the larger fronts in the column sweeps.
 static const int64_t SV_MAXDIM = 768, SV_MAXNP = 64, SV_MAXBLK = 32768;
+// front fi's packed pieces (k_front_pack): their offsets from *size on, which moves past them, and the rows of its L pieces
+static void pack_layout(const FrontPlan &P, const DevPlan &D, int64_t fi, long long *u_pk, long long *l_pk, long long *l_rows, int64_t *size)
+{
+    const Front &F = P.fronts[(size_t)fi];
+    const int64_t np = std::min(F.npiv, F.nrows), nb = (np + 15) / 16, R = D.chain_begin >= 0 && fi >= D.chain_begin ? F.nrows : np;
+    *u_pk = *size;
+    *l_pk = *size + pk_u(nb);
+    *l_rows = R;
+    *size = *l_pk + (nb > 0 ? pk_l(nb - 1, R) + 256 + 16 * (R - np) : 0);
+}
+
 static int upload_solve_levels(const FrontPlan &P, DevPlan &D, char *err, size_t errlen)
 {
     const int64_t nf = (int64_t)P.fronts.size(), nlev = P.nlevels > 0 ? P.nlevels : 1;
     std::vector<SvFront> sv((size_t)(nf > 0 ? nf : 1));
     std::vector<std::vector<int64_t>> lr((size_t)nlev), lc((size_t)nlev);
+    std::vector<int> dfront;
+    D.dblk = 0; D.pk_size = 0;
     D.big_rows.assign((size_t)nlev, {});
     D.big_cols.assign((size_t)nlev, {});
     D.sv_rows_maxnr.assign((size_t)nlev, 0); D.sv_rows_maxnp.assign((size_t)nlev, 0);
     D.sv_cols_maxnc.assign((size_t)nlev, 0); D.sv_cols_maxnp.assign((size_t)nlev, 0);
     for (int64_t fi = 0; fi < nf; fi++) {
         const Front &F = P.fronts[fi];
-        sv[(size_t)fi] = SvFront{F.f, F.npiv, F.nrows, F.nri, F.ncols, F.L_off, F.U_off, F.row_off, F.col_off, 0, 0};
+        sv[(size_t)fi] = SvFront{F.f, F.npiv, F.nrows, F.nri, F.ncols, F.L_off, F.U_off, F.row_off, F.col_off, 0, 0, D.dblk, 0, 0, 0};
+        pack_layout(P, D, fi, &sv[(size_t)fi].u_pk, &sv[(size_t)fi].l_pk, &sv[(size_t)fi].l_rows, &D.pk_size);
+        for (int64_t b = 0; b < (std::min(F.npiv, F.nrows) + 15) / 16; b++) dfront.push_back((int)fi);
+        D.dblk = (int64_t)dfront.size();
         const size_t L = (size_t)F.level;
         const int64_t ncb = F.ncols - F.npiv;
         const bool base = F.npiv <= SV_MAXNP && F.npiv <= F.nrows;
@@ -138,8 +157,8 @@ static int upload_solve_levels(const FrontPlan &P, DevPlan &D, char *err, size_t
             D.sv_cols_maxnp[L] = std::max(D.sv_cols_maxnp[L], F.npiv);
         } else D.big_cols[L].push_back(fi);
     }
-    // the larger fronts of the trans-0 sweeps: device lists by level; the U sweep's CB-column chunks (at most 296, at least
-    // 32 columns each) and each front's first partial sum within its level
+    // the larger fronts of the trans-0 sweeps: device lists by level; the U sweep's CB-column chunks (at most 148, at least
+    // 128 columns each: fewer partial sums for the front's CTA to add) and each front's first partial sum within its level
     std::vector<int> brows_list, bcols_list;
     D.sv_brows_ptr.assign(1, 0); D.sv_bcols_ptr.assign(1, 0);
     D.brows_maxnr.assign((size_t)nlev, 0); D.brows_maxnp.assign((size_t)nlev, 0); D.brows_maxm.assign((size_t)nlev, 0);
@@ -160,7 +179,7 @@ static int upload_solve_levels(const FrontPlan &P, DevPlan &D, char *err, size_t
             const Front &F = P.fronts[(size_t)fi];
             if (F.npiv == 0 || (D.chain_begin >= 0 && fi >= D.chain_begin)) continue;
             const int64_t ncb = F.ncols - F.npiv;
-            const int64_t chunk = ncb > 0 ? std::max<int64_t>(32, (ncb + 295) / 296) : 1;
+            const int64_t chunk = ncb > 0 ? std::max<int64_t>(128, (ncb + 147) / 148) : 1;
             const int64_t nch = ncb > 0 ? (ncb + chunk - 1) / chunk : 0;
             sv[(size_t)fi].nch = nch;
             sv[(size_t)fi].poff = poff;
@@ -217,6 +236,8 @@ static int upload_solve_levels(const FrontPlan &P, DevPlan &D, char *err, size_t
     std::vector<int64_t> iota((size_t)std::max<int64_t>(1, P.max_nrows));
     for (size_t i = 0; i < iota.size(); i++) iota[i] = (int64_t)i;
     int rc;
+    if (dfront.empty()) dfront.push_back(0);
+    if ((rc = upload(dfront, &D.dfront, err, errlen))) return rc;
     if ((rc = upload(sv, &D.sv, err, errlen))) return rc;
     if ((rc = upload(rows_list, &D.sv_rows, err, errlen))) return rc;
     if ((rc = upload(brows_list, &D.sv_brows, err, errlen))) return rc;
@@ -295,6 +316,7 @@ static int upload_batched_fronts(const FrontPlan &P, DevPlan &D, char *err, size
 int dev_upload_plan(const fplus_symbolic *S, const FrontPlan &P, DevPlan &D, char *err, size_t errlen)
 {
     CK(cudaGetDevice(&D.device));
+    CK(cudaDeviceGetAttribute(&D.sms, cudaDevAttrMultiProcessorCount, D.device));
     int rc;
     if ((rc = upload(P.cols, &D.cols, err, errlen))) return rc;
     if ((rc = upload(P.relcol, &D.relcol, err, errlen))) return rc;
@@ -324,6 +346,35 @@ int dev_upload_plan(const fplus_symbolic *S, const FrontPlan &P, DevPlan &D, cha
         if (ok) {
             D.chain_begin = c0; D.chain_nb = nb; D.chain_f0 = P.fronts[c0].f;
             if ((rc = upload(uoff, &D.chain_uoff, err, errlen))) return rc;
+            // the chain as the one-launch sweeps take it (chain_solve.cuh): every front but the first with the one before
+            // as its only child, the row vector of a front in one CTA
+            std::vector<ChainFront> cf;
+            bool one = true, uo_ok = nb % 2 == 0;
+            int64_t u_next = P.fronts[c0].U_off;
+            int64_t mnr = 0, pks = 0;
+            long long up = 0, lp = 0, lr = 0;
+            D.chain_begin = c0;
+            for (int64_t j = 0; j < c0; j++) pack_layout(P, D, j, &up, &lp, &lr, &pks);
+            for (int64_t j = c0; one && j < nf; j++) {
+                const Front &F = P.fronts[j];
+                pack_layout(P, D, j, &up, &lp, &lr, &pks);
+                ChainFront c = {F.f, F.npiv, F.nrows, F.row_off, 0, 0, 0, up, lp};
+                // (U12 blocks one after another, as the column sweep finds them)
+                uo_ok = uo_ok && F.U_off == u_next;
+                u_next += F.npiv * (F.ncols - F.npiv);
+                if (j > c0) {
+                    const Front &G = P.fronts[j - 1];
+                    one = F.child_end - F.child_begin == 1 && P.children[(size_t)F.child_begin] == j - 1;
+                    c.nslot = std::max<int64_t>(0, G.nri - G.npiv); c.slot = G.slot; c.tau = F.tau_base;
+                }
+                one = one && F.nrows <= CH_MAXNR && F.nri == F.nrows && (j + 1 < nf || F.nrows == F.npiv);
+                mnr = std::max(mnr, F.nrows);
+                cf.push_back(c);
+            }
+            if (one && uo_ok && chain_l_smem(mnr, 1, 16) <= 220 * 1024) {
+                D.ch_count = nf - c0; D.ch_maxnr = mnr; D.ch_u0 = P.fronts[c0].U_off; D.ch_nplast = P.fronts[nf - 1].npiv;
+                if ((rc = upload(cf, &D.ch_fronts, err, errlen))) return rc;
+            }
         }
     }
     if ((rc = upload_solve_levels(P, D, err, errlen))) return rc;
@@ -338,7 +389,7 @@ DevNum::~DevNum()
                     (void *)cbstack, (void *)work, (void *)rowid, (void *)p_lu, (void *)pinv, (void *)ipiv, (void *)perm,
                     (void *)st, (void *)scratch, (void *)rbuf, (void *)sbuf, (void *)xbuf, (void *)part, (void *)work2,
                     (void *)perm2, (void *)rr_p, (void *)rr_l, (void *)rr_s, (void *)ir_b, (void *)ir_x, (void *)ir_r,
-                    (void *)ir_d, (void *)ir_bits, scratch_norm, tcws, gm_buf, coopbuf, (void *)permall, vbuf, bsw, bscb})
+                    (void *)ir_d, (void *)ir_bits, scratch_norm, tcws, gm_buf, coopbuf, (void *)permall, vbuf, bsw, bscb, pk, (void *)chsync, chacc})
         if (p) cudaFreeAsync(p, stream);
     if (stream) cudaStreamSynchronize(stream);
     if (crit) cudaStreamSynchronize(crit);
@@ -551,7 +602,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
     int rc;
     *border_front = -1;
     if ((rc = ensure_async(N, (void **)&N.Larena, &N.cap_L, (size_t)P.L_size * vs, err, errlen))) return rc;
-    if ((rc = ensure_async(N, (void **)&N.Uarena, &N.cap_U, (size_t)P.U_size * vs, err, errlen))) return rc;
+    if ((rc = ensure_async(N, (void **)&N.Uarena, &N.cap_U, (size_t)P.U_size * vs + 32, err, errlen))) return rc;
     if ((rc = ensure_async(N, (void **)&N.cbstack, &N.cap_cb, (size_t)P.cb_size * vs, err, errlen))) return rc;
     if ((rc = ensure_async(N, (void **)&N.work, &N.cap_work, (size_t)P.work_size * vs, err, errlen))) return rc;
     if ((rc = ensure_async(N, (void **)&N.rowid, &N.cap_rowid, (size_t)P.rows_total * 8, err, errlen))) return rc;
@@ -591,25 +642,23 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
         int dev = 0, sms = 0, k = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaFuncSetAttribute(k_block_lu_mc<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_block_lu_mc<T, false>, MC_THREADS, mc_smem<T>(per_max, false)) != cudaSuccess)
+        if (cudaFuncSetAttribute(k_block_lu_mc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_block_lu_mc<T>, MC_THREADS, mc_smem<T>(per_max)) != cudaSuccess)
             k = 0;
         (void)cudaGetLastError();
         mc_sms = k >= 1 ? sms : 0;
         // the largest cluster the device places with the cluster form's largest shared memory
-        // (the opt-in is the largest request of the cluster form: with the 220 KB cap its static posts would pass the 227 KB
-        // limit for complex values)
-        if (cudaFuncSetAttribute(k_block_lu_mc<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mc_smem<T>(per_max, true)) == cudaSuccess &&
-            cudaFuncSetAttribute(k_block_lu_mc<T, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-            for (int csz = MC_CMAX; csz >= 4 && mc_cl == 0; csz /= 2) {
+        if (cudaFuncSetAttribute(k_block_lu_cl<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl_smem<T>(per_max)) == cudaSuccess &&
+            cudaFuncSetAttribute(k_block_lu_cl<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            for (int csz = CL_MAXG; csz >= 4 && mc_cl == 0; csz /= 2) {
                 cudaLaunchConfig_t oc = {};
                 cudaLaunchAttribute at[1];
                 at[0].id = cudaLaunchAttributeClusterDimension;
                 at[0].val.clusterDim.x = (unsigned)csz; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                oc.gridDim = dim3((unsigned)csz); oc.blockDim = dim3(MC_THREADS); oc.dynamicSmemBytes = mc_smem<T>(per_max, true);
+                oc.gridDim = dim3((unsigned)csz); oc.blockDim = dim3((unsigned)std::max(256, per_max)); oc.dynamicSmemBytes = cl_smem<T>(per_max);
                 oc.attrs = at; oc.numAttrs = 1;
                 int ncl = 0;
-                if (cudaOccupancyMaxActiveClusters(&ncl, (const void *)k_block_lu_mc<T, true>, &oc) == cudaSuccess && ncl >= 1) mc_cl = csz;
+                if (cudaOccupancyMaxActiveClusters(&ncl, (const void *)k_block_lu_cl<T>, &oc) == cudaSuccess && ncl >= 1) mc_cl = csz;
             }
         }
         (void)cudaGetLastError();
@@ -620,8 +669,13 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
                  mc_ub = r256((size_t)(P.max_npiv > 0 ? P.max_npiv : 1) * (P.max_npiv > 0 ? P.max_npiv : 1) * vs),
                  mc_mark = r256((size_t)(P.max_nrows > 0 ? P.max_nrows : 1) * 4), mc_rid = r256((size_t)(P.max_nrows > 0 ? P.max_nrows : 1) * 8);
     bool any_mc = false;
+    // the cluster form also takes the blocks that one CTA holds but the panel LU does not (300 and more rows of 64 columns):
+    // a step costs 0.6 us there against 2 us and more in k_front_lu2
+    auto takes_mc = [&](int64_t nr, int64_t np) {
+        return front_lu_smem(nr, np, vs) > SMEM_MAX || ((N.lu_variant & 7) == 2 && mc_cl > 0 && !front_lu6_fits<T>(nr, np) && nr >= np && np > 0 && nr >= 64);
+    };
     for (const Front &F : P.fronts)
-        if (front_lu_smem(F.nrows, F.npiv, vs) > SMEM_MAX) { any_mc = true; break; }
+        if (takes_mc(F.nrows, F.npiv)) { any_mc = true; break; }
     any_mc = any_mc && (mc_sms > 0 || mc_cl > 0);
     if (any_mc) {
         if ((rc = ensure_async(N, &N.coopbuf, &N.cap_coop, mc_slots + mc_tk + mc_ch + mc_ub + mc_mark + mc_rid, err, errlen))) return rc;
@@ -650,7 +704,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
     for (int64_t fi = 0; fi < nf; fi++) {
         const Front &F = P.fronts[fi];
         const int64_t nr = F.nrows, np = F.npiv, ncb = F.ncols - F.npiv;
-        bool ok = F.dense && np > 0 && np <= nr && np <= FT_NP && nr <= FT_NR && front_lu_smem(nr, np, vs) <= SMEM_MAX;
+        bool ok = F.dense && np > 0 && np <= nr && np <= FT_NP && nr <= FT_NR && front_lu_smem(nr, np, vs) <= SMEM_MAX && !takes_mc(nr, np);
         ok = ok && (ncb == 0 || (F.parent == fi + 1 && hc[fi] >= 0));
         for (int64_t k = F.child_begin; ok && k < F.child_end; k++) ok = hc[P.children[k]] >= 0;
         pipe[fi] = ok;
@@ -747,7 +801,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
         {
             double fl = 0;
             for (int64_t k = 0; k < std::min(np, nr); k++) fl += (double)(nr - k - 1) * (double)(np - k);
-            prof.begin(st, sm <= SMEM_MAX ? PROF_LU : PROF_LU_TALL, fm * fl, 2.0 * (double)(nr * np) * vs);
+            prof.begin(st, takes_mc(nr, np) ? PROF_LU_TALL : PROF_LU, fm * fl, 2.0 * (double)(nr * np) * vs);
         }
         if ((N.lu_variant & 3) == 3 && use_lu3(nr, np, vs)) {
             const size_t sm3 = front_lu3_smem(nr, np, vs);
@@ -771,7 +825,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             } else
                 lu6<<<1, nt6, sm6, st>>>(W, ld, (int)nr, (int)np, (int)F.nri, F.f, N.colmax, pivot_rel, N.rowid + F.row_off, Lf, perm,
                                          N.p_lu, N.st, fi, pa), note_launch();
-        } else if (sm <= SMEM_MAX) {
+        } else if (sm <= SMEM_MAX && !takes_mc(nr, np)) {
             const int R = (int)((nr + 31) & ~31);
             int nt = 32 + (R <= 128 ? 4 * R : R);   // the pivot warp + the update warps
             if (nt > 640) nt = 640;
@@ -788,9 +842,9 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             // when it holds them, else a cooperative launch
             bool done = false;
             if (any_mc && !(N.lu_variant & 4)) {
-                // (measured on B200: the cluster form is the faster up to about 3,000 rows, with as many CTAs as the
-                // cluster takes; above, the grid form over the SMs)
-                const bool cl = mc_cl > 0 && nr <= std::min<int64_t>((int64_t)mc_cl * per_max, 3072);
+                // (the cluster form as far as its CTAs hold the rows, with as many CTAs as the cluster takes; above, the
+                // grid form over the SMs: a step of it costs about 4 us, a global round trip, against 0.6 us)
+                const bool cl = mc_cl > 0 && nr <= (int64_t)mc_cl * per_max;
                 int G = cl ? (int)std::min<int64_t>(mc_cl, std::max<int64_t>(2, (nr + 31) / 32))
                            : (int)std::min<int64_t>(mc_sms, std::max<int64_t>(1, (nr + 63) / 64));
                 if ((nr + G - 1) / G > per_max) G = (int)((nr + per_max - 1) / per_max);
@@ -802,10 +856,10 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
                     cudaLaunchAttribute at[1];
                     at[0].id = cudaLaunchAttributeClusterDimension;
                     at[0].val.clusterDim.x = (unsigned)G; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                    cfg.gridDim = dim3((unsigned)G); cfg.blockDim = dim3(MC_THREADS); cfg.dynamicSmemBytes = mc_smem<T>(per, true);
+                    cfg.gridDim = dim3((unsigned)G); cfg.blockDim = dim3((unsigned)std::max(256, (per + 31) & ~31)); cfg.dynamicSmemBytes = cl_smem<T>(per);
                     cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
-                    le = cudaLaunchKernelEx(&cfg, k_block_lu_mc<T, true>, W, ld, (int)nr, (int)np, (int)F.nri, per, F.f,
-                                            (const double *)N.colmax, pivot_rel, rid, mc_chosen, mc_U, mc_slot, mc_sync, N.st, fi);
+                    le = cudaLaunchKernelEx(&cfg, k_block_lu_cl<T>, W, ld, (int)nr, (int)np, (int)F.nri, per, F.f,
+                                            (const double *)N.colmax, pivot_rel, rid, mc_chosen, mc_U, N.st, fi);
                 } else if (!cl && mc_sms > 0 && G <= mc_sms) {
                     T *Wp = W;
                     int64_t ldl = ld, fcol = F.f, frow = fi;
@@ -818,8 +872,8 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
                     unsigned int *sy = mc_sync;
                     DevStatus *stp = N.st;
                     void *args[] = {&Wp, &ldl, &nri_, &npi, &nrii, &peri, &fcol, &cm, &prel, &rid, &chs, &ub, &sl, &sy, &stp, &frow};
-                    le = cudaLaunchCooperativeKernel((const void *)k_block_lu_mc<T, false>, G, MC_THREADS, args,
-                                                     mc_smem<T>(per, false), st);
+                    le = cudaLaunchCooperativeKernel((const void *)k_block_lu_mc<T>, G, MC_THREADS, args,
+                                                     mc_smem<T>(per), st);
                 }
                 if (le == cudaSuccess) {
                     note_launch();
@@ -1095,6 +1149,10 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
     if (in_pipe) { CK(cudaEventRecord(N.ev_lu, A)); CK(cudaStreamWaitEvent(s, N.ev_lu, 0)); }    // the bulk stream joins
     CK(cudaGetLastError());
     k_pinv<<<nblk(N.n), 256, 0, s>>>(N.p_lu, N.pinv, N.n, N.st), note_launch();
+    if (D.dblk > 0) {                    // the packed triangles, for the sweeps
+        if ((rc = ensure_async(N, &N.pk, &N.cap_pk, (size_t)D.pk_size * vs, err, errlen))) return rc;
+        k_front_pack<T><<<(unsigned)D.dblk, 128, 0, s>>>(D.sv, D.dfront, La, (T *)N.pk, N.st), note_launch();
+    }
     if (N.capture) return FPLUS_OK;              // the status is read after the graph has run
     DevStatus h;
     CK(cudaMemcpyAsync(&h, N.st, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -1155,6 +1213,85 @@ int dev_factor_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
+// the dense chain's sweeps in one launch each (chain_solve.cuh): L or L^T (row sweep) and U or U^T (column sweep)
+template <typename T, int TR, int RB>
+static int chain_row_sweep(const FrontPlan &P, const DevPlan &D, DevNum &N, const T *VB, const T *R, T *S2, int64_t nrhs,
+                           char *err, size_t errlen)
+{
+    const size_t sm = chain_l_smem(D.ch_maxnr, RB, sizeof(T));
+    CK(cudaFuncSetAttribute(k_chain_l<T, TR, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    const Front &C = P.fronts[(size_t)D.chain_begin];
+    k_chain_l<T, TR, RB><<<(unsigned)((nrhs + RB - 1) / RB), CH_THREADS, sm, N.stream>>>(
+        D.ch_fronts, (int)D.ch_count, (int)D.ch_maxnr, (const T *)N.pk, N.permall, D.rowinit, VB + C.row_off, D.vrow, R, S2, N.n,
+        (int)nrhs, N.st), note_launch();
+    return FPLUS_OK;
+}
+template <typename T, int TR, int RB>
+static int chain_col_sweep(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, int64_t G, char *err, size_t errlen)
+{
+    const int64_t K = D.ch_count, own = (K + G - 2) / (G - 1);
+    const bool wide = chain_u_smem(own, RB, sizeof(T)) > 226 * 1024;     // (the workers' sums in global memory)
+    const size_t sm = chain_u_smem(wide ? 0 : own, RB, sizeof(T));
+    int rc;
+    if (wide && (rc = ensure_async(N, &N.chacc, &N.cap_chacc, (size_t)(K * CH_NB * RB) * sizeof(T), err, errlen))) return rc;
+    CK(cudaFuncSetAttribute(k_chain_u<T, TR, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    for (int64_t r0 = 0; r0 < nrhs; r0 += RB) {
+        CK(cudaMemsetAsync(N.chsync, 0, (size_t)(K + 1) * 4, N.stream));
+        const ChainFront *fr = D.ch_fronts;
+        int Ki = (int)K, nb = (int)D.chain_nb, m = (int)std::min<int64_t>(RB, nrhs - r0), npl = (int)D.ch_nplast;
+        const T *Ua = (const T *)N.Uarena, *pk = (const T *)N.pk;
+        T *Yr = Y + r0 * N.n, *Xr = X + r0 * N.n;
+        int64_t n = N.n, f0 = D.chain_f0, U0 = D.ch_u0;
+        unsigned *sy = N.chsync;
+        DevStatus *st = N.st;
+        T *ga = wide ? (T *)N.chacc : nullptr;
+        void *args[] = {&fr, &Ki, &nb, &f0, &U0, &npl, &Ua, &pk, &Yr, &Xr, &n, &m, &sy, &ga, &st};
+        CK(cudaLaunchCooperativeKernel((const void *)k_chain_u<T, TR, RB>, (unsigned)G, CH_UTHREADS, args, sm, N.stream));
+        note_launch();
+    }
+    return FPLUS_OK;
+}
+// the same by a launch per step, for captured graphs
+template <typename T, int TR, int RB>
+static int chain_col_steps(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, char *err, size_t errlen)
+{
+    const int K = (int)D.ch_count;
+    const size_t sm = chain_ustep_smem(RB, sizeof(T));
+    int rc;
+    if ((rc = ensure_async(N, &N.chacc, &N.cap_chacc, (size_t)(D.ch_count * CH_NB * RB) * sizeof(T), err, errlen))) return rc;
+    CK(cudaFuncSetAttribute(k_chain_ustep<T, TR, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    for (int64_t r0 = 0; r0 < nrhs; r0 += RB)
+        for (int s = -1; s < K - 1; s++) {
+            CK(launch_pdl(k_chain_ustep<T, TR, RB>, 1 + std::max(0, s >= 0 ? K - 2 - s : 0), CH_THREADS, sm, N.stream, (const ChainFront *)D.ch_fronts,
+                          K, (int)D.chain_nb, D.chain_f0, D.ch_u0, (int)D.ch_nplast, (const T *)N.Uarena, (const T *)N.pk, Y + r0 * N.n,
+                          X + r0 * N.n, N.n, (int)std::min<int64_t>(RB, nrhs - r0), s, (T *)N.chacc, (const DevStatus *)N.st));
+            note_launch();
+        }
+    return FPLUS_OK;
+}
+// U x = y (TR 0: Y in pivot order, x into X) or U^T z = w (in place).  Workers: one per block as far as the SMs go (one SM
+// takes a 64 KB block in about 1.4 us, more blocks per worker lengthen every step); a launch per step in a captured graph.
+// The result depends on neither.  Right-hand sides per pass over U: ch_rb
+template <typename T, int TR>
+static int chain_columns(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, char *err, size_t errlen)
+{
+    if (N.capture || N.capture_size) {
+        if (nrhs == 1) return chain_col_steps<T, TR, 1>(D, N, Y, X, nrhs, err, errlen);
+        return chain_col_steps<T, TR, ch_rb<T>()>(D, N, Y, X, nrhs, err, errlen);
+    }
+    const int64_t K = D.ch_count, G = 1 + std::max<int64_t>(1, std::min<int64_t>(D.sms - 1, K - 2));
+    int rc;
+    if ((rc = ensure_async(N, (void **)&N.chsync, &N.cap_chsync, (size_t)(K + 1) * 4, err, errlen))) return rc;
+    if (nrhs == 1) return chain_col_sweep<T, TR, 1>(D, N, Y, X, nrhs, G, err, errlen);
+    return chain_col_sweep<T, TR, ch_rb<T>()>(D, N, Y, X, nrhs, G, err, errlen);
+}
+template <typename T, int TR>
+static int chain_rows(const FrontPlan &P, const DevPlan &D, DevNum &N, const T *VB, const T *R, T *S2, int64_t nrhs, char *err, size_t errlen)
+{
+    if (nrhs == 1 || chain_l_smem(D.ch_maxnr, ch_rb<T>(), sizeof(T)) > SMEM_MAX) return chain_row_sweep<T, TR, 1>(P, D, N, VB, R, S2, nrhs, err, errlen);
+    return chain_row_sweep<T, TR, ch_rb<T>()>(P, D, N, VB, R, S2, nrhs, err, errlen);
+}
+
 // solves on device buffers: x (n x nrhs, ld = n) in, solution out, through the plan's fronts
 template <typename T>
 static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *xb, int64_t nrhs, int trans, int raw,
@@ -1189,19 +1326,29 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
     const T *La = (const T *)N.Larena, *Ua = (const T *)N.Uarena;
     const int64_t nf = (int64_t)P.fronts.size();
     const int64_t nlev = (int64_t)D.sv_rows_ptr.size() - 1;
+    // The dense chain's sweeps in one launch each where its fronts qualify (upload_plan) and the block inverses are there;
+    // measured against a launch per front: see the kernels' comments
+    const bool one_chain = D.ch_count > 0;
+    const T *PK = (const T *)N.pk;
+    const int64_t RBS = nrhs == 1 ? 1 : 8;       // right-hand sides per pass of the sweep kernels
+    auto tri_stages = [&](int64_t np) { return tri16_elems(np, RBS, 3) * (int64_t)sizeof(T) <= (int64_t)SMEM_MAX ? 3 : tri16_elems(np, RBS, 2) * (int64_t)sizeof(T) <= (int64_t)SMEM_MAX ? 2 : 0; };
+    const int64_t chain_lv = D.chain_begin >= 0 ? (int64_t)P.fronts[(size_t)D.chain_begin].level : nlev;
     {
         static thread_local bool sv_attr = false;
         if (!sv_attr) {
-            CK(cudaFuncSetAttribute(k_sv_fwdL<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-            CK(cudaFuncSetAttribute(k_sv_bwdU<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+            for (const void *k : {(const void *)k_sw_fwdL<T, 1>, (const void *)k_sw_fwdL<T, 8>, (const void *)k_sw_bwdU<T, 1>,
+                                  (const void *)k_sw_bwdU<T, 8>, (const void *)k_swb_L11<T, 1, 3>, (const void *)k_swb_L11<T, 8, 3>,
+                                  (const void *)k_swb_L11<T, 1, 2>, (const void *)k_swb_L11<T, 8, 2>, (const void *)k_swb_L21<T, 1>,
+                                  (const void *)k_swb_L21<T, 8>, (const void *)k_swb_u12<T, 1>, (const void *)k_swb_u12<T, 8>,
+                                  (const void *)k_swb_bwdU<T, 1, 3>, (const void *)k_swb_bwdU<T, 8, 3>, (const void *)k_swb_bwdU<T, 1, 2>,
+                                  (const void *)k_swb_bwdU<T, 8, 2>})
+                CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_sv_fwdUt<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_sv_fwdUt<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_sv_bwdLt<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_sv_bwdLt<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_svb_L11<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-            CK(cudaFuncSetAttribute(k_svb_L21<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             CK(cudaFuncSetAttribute(k_svb_bwdU<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-            CK(cudaFuncSetAttribute(k_svb_u12<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
             sv_attr = true;
         }
     }
@@ -1235,15 +1382,15 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
         // fronts together (their vectors gathered into VB, then the L11 solves and the L21 products there); y into S2 in
         // pivot order.  The dense chain (the levels above the tree, a front each) sequentially in the row-space vector:
         // its first front's gathered vector into R, then front after front (the next launch overlapping the previous).
-        const int64_t chain_lv = D.chain_begin >= 0 ? (int64_t)P.fronts[(size_t)D.chain_begin].level : nlev;
         for (int64_t lv = 0; lv < chain_lv; lv++) {
             const int64_t a0 = D.sv_rows_ptr[(size_t)lv], a1 = D.sv_rows_ptr[(size_t)lv + 1];
             if (a1 > a0) {
                 const int64_t mnr = D.sv_rows_maxnr[(size_t)lv], mnp = D.sv_rows_maxnp[(size_t)lv];
-                const size_t sm = (size_t)(mnr * SV_RC + mnp * SV_RC + 64 * mnp) * sizeof(T);
-                CK(launch_pdl(k_sv_fwdL<T>, (int)(a1 - a0), SV_THREADS, sm, s, (const SvFront *)D.sv, (const int *)(D.sv_rows + a0),
-                              La, (const int64_t *)D.rowinit, (const int *)N.permall, (const int64_t *)D.rsp,
-                              (const int64_t *)D.rsi, (const T *)R, S2, VB, D.vrow, n, (int)nrhs));
+                const size_t sm = (size_t)sw_fwdL_elems(mnr, mnp, RBS) * sizeof(T);
+                auto kern = nrhs == 1 ? k_sw_fwdL<T, 1> : k_sw_fwdL<T, 8>;
+                CK(launch_pdl(kern, (int)(a1 - a0), SW_THREADS, sm, s, (const SvFront *)D.sv, (const int *)(D.sv_rows + a0),
+                              La, PK, (const int64_t *)D.rowinit, (const int *)N.permall, (const int64_t *)D.rsp,
+                              (const int64_t *)D.rsi, (const T *)R, S2, VB, D.vrow, n, (int)nrhs, N.st));
                 note_launch();
             }
             // the level's larger fronts together: their vectors, the L11 solves (a CTA each), the L21 products
@@ -1257,11 +1404,19 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                 k_svb_gatherL<T><<<dim3(gx, nb), 256, 0, s>>>(D.sv, bl, D.rowinit, N.permall, D.rsp, D.rsi, R, VB, D.vrow, n,
                                                               nrhs), note_launch();
                 if (mnp > 0) {
-                    // the L11 solves: at most 8 right-hand sides per CTA (the groups in parallel)
-                    const int rcb = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nrhs, 8),
-                        (int64_t)((SMEM_MAX - 64 * 64 * sizeof(T)) / ((size_t)mnp * sizeof(T)))));
-                    k_svb_L11<T><<<dim3(nb, (unsigned)((nrhs + rcb - 1) / rcb)), 256, ((size_t)mnp * rcb + 64 * 64) * sizeof(T), s>>>(
-                        D.sv, bl, La, VB, D.vrow, S2, n, (int)nrhs, rcb), note_launch();
+                    // the L11 solves: at most 8 right-hand sides per CTA (the groups in parallel); by 16-column blocks while
+                    // shared memory holds two of them, else (more than 256 complex, 512 real pivots) by 64-row substitution
+                    const int stg = tri_stages(mnp);
+                    if (stg) {
+                        auto kern = nrhs == 1 ? (stg == 3 ? k_swb_L11<T, 1, 3> : k_swb_L11<T, 1, 2>) : (stg == 3 ? k_swb_L11<T, 8, 3> : k_swb_L11<T, 8, 2>);
+                        kern<<<dim3(nb, (unsigned)((nrhs + RBS - 1) / RBS)), SW_THREADS, (size_t)tri16_elems(mnp, RBS, stg) * sizeof(T), s>>>(
+                            D.sv, bl, PK, VB, D.vrow, S2, n, (int)nrhs, N.st), note_launch();
+                    } else {
+                        const int rcb = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nrhs, 8),
+                            (int64_t)((SMEM_MAX - 64 * 64 * sizeof(T)) / ((size_t)mnp * sizeof(T)))));
+                        k_svb_L11<T><<<dim3(nb, (unsigned)((nrhs + rcb - 1) / rcb)), 256, ((size_t)mnp * rcb + 64 * 64) * sizeof(T), s>>>(
+                            D.sv, bl, La, VB, D.vrow, S2, n, (int)nrhs, rcb), note_launch();
+                    }
                     if (mm > 0 && nrhs >= 8 && nb == 1) {
                         // one front and several right-hand sides: u = v[np:] - L21 x as an FP64 tensor-core GEMM, in place
                         const Front &F1 = P.fronts[(size_t)D.sv_brows_host[(size_t)b0]];
@@ -1273,9 +1428,12 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                                                             D.vrow, nullptr, C, D.vrow, N.st, OutMap{}), note_launch();
                         }
                     } else if (mm > 0) {
-                        const int rc2 = (int)std::max<int64_t>(1, std::min<int64_t>(SVB_RC, (int64_t)(SMEM_MAX / ((size_t)mnp * sizeof(T)))));
-                        k_svb_L21<T><<<dim3((unsigned)((mm + 255) / 256), nb), 256, (size_t)mnp * rc2 * sizeof(T), s>>>(
-                            D.sv, bl, La, VB, D.vrow, (int)nrhs, rc2), note_launch();
+                        const size_t sm8 = (size_t)(8 * (mnp + SW_THREADS)) * sizeof(T);
+                        const dim3 g((unsigned)((mm + 31) / 32), nb);
+                        if (nrhs == 1 || sm8 > SMEM_MAX)
+                            k_swb_L21<T, 1><<<g, SW_THREADS, (size_t)(mnp + SW_THREADS) * sizeof(T), s>>>(D.sv, bl, La, VB, D.vrow, (int)nrhs), note_launch();
+                        else
+                            k_swb_L21<T, 8><<<g, SW_THREADS, sm8, s>>>(D.sv, bl, La, VB, D.vrow, (int)nrhs), note_launch();
                     }
                 }
             }
@@ -1285,6 +1443,9 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
             k_sv_gatherL<T><<<nblk(C.nrows * nrhs), 256, 0, s>>>(C.row_off, C.nrows, C.nri, D.rowinit,
                                                                  C.npiv > 0 ? N.permall + C.row_off : nullptr, D.rsp, D.rsi, R, VB,
                                                                  D.vrow, n, nrhs), note_launch();
+            if (one_chain) {
+                if ((rc = chain_rows<T, 0>(P, D, N, VB, R, S2, nrhs, err, errlen))) return rc;
+            } else {
             k_sv_toR<T><<<nblk(C.nrows * nrhs), 256, 0, s>>>(VB + C.row_off, D.vrow, C.nrows, N.rowid + C.row_off, R, n, nrhs),
                 note_launch();
             for (int64_t fi = D.chain_begin; fi < nf; fi++) {
@@ -1311,9 +1472,11 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                     k_fwdL<T><<<1, 256, 0, s>>>(La + F.L_off, F.nrows, F.npiv, N.rowid + F.row_off, R, n, nrhs), note_launch();
             }
             k_gather_range<T><<<nblk((n - C.f) * nrhs), 256, 0, s>>>(S2, R, N.p_lu, C.f, n, nrhs), note_launch();
+            }
         }
-        int64_t fi_end = nf;                   // fronts below the chain: the row-oriented kernel
-        if (D.chain_begin >= 0) {
+        if (one_chain) {
+            if ((rc = chain_columns<T, 0>(D, N, S2, R, nrhs, err, errlen))) return rc;
+        } else if (D.chain_begin >= 0) {
             // the dense chain, column-oriented: front k's launch first applies front k + 1's solution to the rows above
             const int64_t cb = D.chain_begin, nb = D.chain_nb;
             const size_t csm = std::max((size_t)(nb + (nb + 15) / 16) * nrhs, (size_t)(nb * (nrhs + 1) + nb * nb)) * sizeof(T);
@@ -1331,7 +1494,6 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                               jk1, npk1, (const T *)(La + F.L_off), F.nrows, F.f, (int)F.npiv, S2, R, n, nrhs, N.st));
                 note_launch();
             }
-            fi_end = cb;
         }
         CK(cudaFuncSetAttribute(k_bwdU_blk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM));
         // the U sweep below the chain by levels (roots first): the level's small fronts in one launch (a CTA each), then
@@ -1340,9 +1502,10 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
             const int64_t a0 = D.sv_cols_ptr[(size_t)lv], a1 = D.sv_cols_ptr[(size_t)lv + 1];
             if (a1 > a0) {
                 const int64_t mnp = D.sv_cols_maxnp[(size_t)lv];
-                const size_t sm = (size_t)(mnp * SV_RC + 64 * mnp + 64) * sizeof(T);
-                CK(launch_pdl(k_sv_bwdU<T>, (int)(a1 - a0), SV_THREADS, sm, s, (const SvFront *)D.sv, (const int *)(D.sv_cols + a0),
-                              La, Ua, (const int64_t *)D.cols, (const T *)S2, R, n, (int)nrhs, N.st));
+                const size_t sm = (size_t)sw_bwdU_elems(D.sv_cols_maxnc[(size_t)lv], mnp, RBS) * sizeof(T);
+                auto kern = nrhs == 1 ? k_sw_bwdU<T, 1> : k_sw_bwdU<T, 8>;
+                CK(launch_pdl(kern, (int)(a1 - a0), SW_THREADS, sm, s, (const SvFront *)D.sv, (const int *)(D.sv_cols + a0),
+                              La, Ua, PK, (const int64_t *)D.cols, (const T *)S2, R, n, (int)nrhs, N.st));
                 note_launch();
             }
             // the level's larger fronts together: the U12 partial products, then the U11 solves (a CTA each)
@@ -1352,21 +1515,26 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                 const int *bl = D.sv_bcols + b0;
                 const int64_t mnp = D.bcols_maxnp[(size_t)lv], mch = D.bcols_maxnch[(size_t)lv];
                 if (mch > 0) {
-                    const size_t xsm = (size_t)D.bcols_maxchunk[(size_t)lv] * SVB_RC * sizeof(T);
-                    k_svb_u12<T><<<dim3((unsigned)mch, nb), 256, xsm, s>>>(D.sv, bl, Ua, D.cols, R, n, (int)nrhs, part), note_launch();
+                    const size_t xsm = (size_t)RBS * (size_t)(D.bcols_maxchunk[(size_t)lv] + SW_THREADS) * sizeof(T);
+                    auto kern = nrhs == 1 ? k_swb_u12<T, 1> : k_swb_u12<T, 8>;
+                    kern<<<dim3((unsigned)mch, nb, (unsigned)((mnp + 63) / 64)), SW_THREADS, xsm, s>>>(D.sv, bl, Ua, D.cols, R, n, (int)nrhs, part), note_launch();
                     // the partial sums over many CTAs when a front's right-hand sides are more than its CTA's threads
                     if (mnp * nrhs > 256) {
                         const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>((mnp * nrhs + 255) / 256, 148));
                         k_svb_psum<T><<<dim3(gx, nb), 256, 0, s>>>(D.sv, bl, part, S2, n, (int)nrhs), note_launch();
                     }
                 }
-                const int rcb = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nrhs, 8),
-                    (int64_t)((SMEM_MAX - (64 * 64 + 64) * sizeof(T)) / ((size_t)mnp * sizeof(T)))));
-                k_svb_bwdU<T><<<dim3(nb, (unsigned)((nrhs + rcb - 1) / rcb)), 256, ((size_t)mnp * rcb + 64 * 64 + 64) * sizeof(T), s>>>(
-                    D.sv, bl, La, part, S2, R, n,
-                                                                                               (int)nrhs, rcb, N.st,
-                                                                                               mch > 0 && mnp * nrhs > 256 ? 1 : 0),
-                    note_launch();
+                const int pre = mch > 0 && mnp * nrhs > 256 ? 1 : 0, stg = tri_stages(mnp);
+                if (stg) {
+                    auto kern = nrhs == 1 ? (stg == 3 ? k_swb_bwdU<T, 1, 3> : k_swb_bwdU<T, 1, 2>) : (stg == 3 ? k_swb_bwdU<T, 8, 3> : k_swb_bwdU<T, 8, 2>);
+                    kern<<<dim3(nb, (unsigned)((nrhs + RBS - 1) / RBS)), SW_THREADS, (size_t)tri16_elems(mnp, RBS, stg) * sizeof(T), s>>>(
+                        D.sv, bl, PK, part, S2, R, n, (int)nrhs, pre, N.st), note_launch();
+                } else {
+                    const int rcb = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nrhs, 8),
+                        (int64_t)((SMEM_MAX - (64 * 64 + 64) * sizeof(T)) / ((size_t)mnp * sizeof(T)))));
+                    k_svb_bwdU<T><<<dim3(nb, (unsigned)((nrhs + rcb - 1) / rcb)), 256, ((size_t)mnp * rcb + 64 * 64 + 64) * sizeof(T), s>>>(
+                        D.sv, bl, La, part, S2, R, n, (int)nrhs, rcb, N.st, pre), note_launch();
+                }
             }
         }
         // x[col_perm[k]] = Dcp[k] * R[k]  (raw: x[k] = R[k])
@@ -1379,7 +1547,8 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
         const bool cj = trans == 2;
         // the U^T sweep by levels (leaves first): the level's small fronts in one launch, the others front by front (their
         // column vector gathered: the pivot columns into R, the others into VB; the U11^T solve in R; the contribution)
-        for (int64_t lv = 0; lv < nlev; lv++) {
+        const int64_t lv_end = one_chain ? chain_lv : nlev;
+        for (int64_t lv = 0; lv < lv_end; lv++) {
             const int64_t a0 = D.sv_cols_ptr[(size_t)lv], a1 = D.sv_cols_ptr[(size_t)lv + 1];
             if (a1 > a0) {
                 const int64_t mnc = D.sv_cols_maxnc[(size_t)lv], mnp = D.sv_cols_maxnp[(size_t)lv];
@@ -1413,8 +1582,17 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                 }
             }
         }
+        if (one_chain) {
+            // the chain's columns, each with the contributions below it, in R; then its two sweeps
+            const Front &C = P.fronts[(size_t)D.chain_begin];
+            k_sv_gatherU<T><<<nblk(C.ncols * nrhs), 256, 0, s>>>(C.f, C.ncols, C.ncols, C.col_off, D.csp, D.csi, R, VB, D.vcol, n, nrhs),
+                note_launch();
+            rc = cj ? chain_columns<T, 2>(D, N, R, R, nrhs, err, errlen) : chain_columns<T, 1>(D, N, R, R, nrhs, err, errlen);
+            if (rc == FPLUS_OK) rc = cj ? chain_rows<T, 2>(P, D, N, VB, R, S2, nrhs, err, errlen) : chain_rows<T, 1>(P, D, N, VB, R, S2, nrhs, err, errlen);
+            if (rc) return rc;
+        }
         // the L^T sweep by levels (roots first): the level's small fronts in one launch, the others front by front
-        for (int64_t lv = nlev - 1; lv >= 0; lv--) {
+        for (int64_t lv = lv_end - 1; lv >= 0; lv--) {
             const int64_t a0 = D.sv_rows_ptr[(size_t)lv], a1 = D.sv_rows_ptr[(size_t)lv + 1];
             if (a1 > a0) {
                 const int64_t mnp = D.sv_rows_maxnp[(size_t)lv];
@@ -1654,6 +1832,7 @@ int dev_status(DevNum &N, int *code, int64_t *idx, char *err, size_t errlen)
     DevStatus h;
     CK(cudaMemcpyAsync(&h, N.st, sizeof(h), cudaMemcpyDeviceToHost, N.stream));
     CK(cudaStreamSynchronize(N.stream));
+    if (h.code == ST_WAIT) { errf(err, errlen, "a wait between the CTAs of one kernel ran out (block %ld)", (long)h.idx); return FPLUS_ERR_GPU; }
     *code = h.code; *idx = h.idx;
     return FPLUS_OK;
 }

@@ -10,6 +10,7 @@
 namespace fpl {
 
 struct DevStatus;
+struct ChainFront;
 
 // per-class device timing (fplus_b200_profile): 0 Schur GEMM into the CB, 1 pivot-block LU, 2 U12 (gather + TRSM),
 // 3 assembly and extend-add
@@ -34,11 +35,17 @@ struct DevPlan {
     // (the last one at most), first column chain_f0, their U offsets; chain_begin < 0 when the fronts do not qualify
     int64_t chain_begin = -1, chain_nb = 0, chain_f0 = 0;
     int64_t *chain_uoff = nullptr;
+    // the chain's fronts for the one-launch sweeps (chain_solve.cuh; ch_count 0: they do not qualify), their most rows
+    ChainFront *ch_fronts = nullptr;
+    int64_t ch_count = 0, ch_maxnr = 0, ch_u0 = 0, ch_nplast = 0;
+    int sms = 148;
     // the level-scheduled solve: every front's descriptor; per level (ascending height) the fronts the one-CTA kernels
     // take, as device lists (sv_rows: the L and L^T sweeps; sv_cols: the U and U^T sweeps) with host ranges and the
     // level's largest sizes, and the others as host lists; the lists of the children's contribution entries landing on
     // each plan row (rsp/rsi) and plan column (csp/csi); 0 .. max_nrows - 1
     SvFront *sv = nullptr;
+    int *dfront = nullptr;         // the front of each 16 x 16 diagonal block (dblk blocks, in the fronts' order)
+    int64_t dblk = 0, pk_size = 0; // (pk_size: the packed triangles' elements)
     int *sv_rows = nullptr, *sv_cols = nullptr;
     std::vector<int64_t> sv_rows_ptr, sv_cols_ptr;
     std::vector<int64_t> sv_rows_maxnr, sv_rows_maxnp, sv_cols_maxnc, sv_cols_maxnp;
@@ -88,6 +95,10 @@ struct DevNum {
     size_t cap_perm = 0;
     int *permall = nullptr;        // every front's final row order (position -> initial local row), kept for the solves
     size_t cap_permall = 0;
+    void *pk = nullptr;            // the fronts' packed triangles with inverted 16 x 16 diagonal blocks (k_front_pack)
+    unsigned *chsync = nullptr;    // the dense chain's sweeps' counters, its workers' sums
+    void *chacc = nullptr;
+    size_t cap_pk = 0, cap_chsync = 0, cap_chacc = 0;
     void *vbuf = nullptr;          // the level-scheduled solve's contribution vectors
     size_t cap_vb = 0;
     void *bsw = nullptr, *bscb = nullptr;   // the batched fronts' working blocks (one level) and contribution blocks
@@ -114,6 +125,7 @@ struct DevNum {
                                    // + 32: the pipelined chain's contribution blocks through the stack and the
                                    // extend-add instead of straight into the parent's working block
     int capture = 0;               // the launches are being captured into a CUDA graph: no host copies, waits or decisions
+    int capture_size = 0;          // an uncaptured solve that sizes the buffers of a captured one
     void *gm_buf = nullptr;        // GMRES-IR: the Krylov basis and its vectors
     size_t cap_gm = 0;
     void *tcws = nullptr;

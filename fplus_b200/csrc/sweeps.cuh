@@ -6,97 +6,103 @@ namespace fpl {
 
 constexpr int SW_THREADS = 256;
 
-// A front's triangle applied to the vector x (np x rc, ld np, shared memory; overwritten as scratch), the result in xs (the
-// same layout): xs = L11^-1 x (UPPER false) or U11^-1 x.  By 16-column blocks: the block's 16 unknowns as one product with
-// the inverted diagonal block (dv: the front's blocks of k_front_dinv), then the rows beyond it updated from the block's
-// columns, which stream through a ring of STG pieces in shared memory (16 np + 256 elements each) ahead of the chain.  One
-// CTA of SW_THREADS; ends with a barrier.
+// A front's triangle applied to the vector x (x[k * RB + r], k up to np and zero from there to the next sixteen, shared
+// memory; overwritten), the result in xs (the same layout): xs = L11^-1 x (UPPER false) or U11^-1 x.  By 16-column blocks: the
+// block's 16 unknowns as one product with the inverted diagonal block, then the rows beyond it updated from the block's
+// columns; the packed pieces (at pk, see k_front_pack) stream through a ring of STG stages of psz elements by bulk copies
+// ahead of the chain.  The pipe (its barriers, initialised, and the pieces taken so far) serves several calls of a CTA of
+// SW_THREADS.  Ends with a barrier; false (for every thread) when a copy did not land.
 //
-// What bounds it: np / 16 dependent block steps of about 450 cycles (two products, two barriers); a 256 x 256 triangle
-// takes about 5 us against 45 us for 64-step substitutions with the triangle read from global memory in between.
+// What bounds it: np / 16 dependent block steps (two small products, two barriers).
+struct TriPipe { unsigned long long *bars; int done; };
+__host__ __device__ constexpr int tri_pad(int np) { return (np + 15) & ~15; }
 template <typename T, bool UPPER, int RB, int STG>
-__device__ __forceinline__ void tri16(const T *__restrict__ L, int64_t ld, int np, T *x, T *xs, int rc, const T *__restrict__ dv, T *ring)
+__device__ __forceinline__ bool tri16(const T *__restrict__ pk, int np, T *x, T *xs, T *ring, int psz, TriPipe &pipe)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nbk = (np + 15) >> 4, psz = 16 * np + 256;
-    int nextb = 0;
+    const int tid = threadIdx.x, nbk = (np + 15) >> 4;
+    int issued = 0;
     auto blk = [&](int i) -> int { return UPPER ? nbk - 1 - i : i; };
-    auto load_next = [&](int slot) {
-        if (nextb < nbk) {
-            const int b = blk(nextb), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16;
-            T *d = ring + slot * psz;
-            const int ra = UPPER ? 0 : k0 + w, re = UPPER ? k0 : np;
-            for (int c = warp; c < w; c += SW_THREADS / 32)
-                for (int row = ra + lane; row < re; row += 32) cp_async_el(d + c * np + row, L + row + (int64_t)(k0 + c) * ld);
-            cp_async_el(d + 16 * np + tid, dv + (int64_t)b * 512 + (UPPER ? 0 : 256) + tid);
-            nextb++;
-        }
-        cp_async_commit();
+    auto load_next = [&]() {                           // one thread
+        if (issued >= nbk) return;
+        const int b = blk(issued), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16, sl = (pipe.done + issued) % STG;
+        const unsigned bytes = (unsigned)((256 + 16 * (UPPER ? k0 : np - k0 - w)) * sizeof(T));
+        bulk_expect(pipe.bars + sl, bytes);
+        bulk_load(ring + sl * psz, pk + (UPPER ? pk_u(b) : pk_l(b, np)), bytes, pipe.bars + sl);
+        issued++;
     };
-#pragma unroll
-    for (int k = 0; k < STG - 1; k++) load_next(k);
-    int slot = 0;
+    if (tid == SW_THREADS - 1) for (int k = 0; k < STG - 1; k++) load_next();
+    bool ok = true;
     for (int i = 0; i < nbk; i++) {
-        const int b = blk(i), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16;
-        cp_async_wait_n<STG - 2>();
-        __syncthreads();
-        load_next((slot + STG - 1) % STG);
-        const T *Lp = ring + slot * psz;
-        slot = (slot + 1) % STG;
+        const int b = blk(i), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16, d = pipe.done + i;
+        ok = bar_wait(pipe.bars + d % STG, (unsigned)(d / STG) & 1u) && ok;
+        __syncthreads();                               // (the piece before is no longer read; x is as its updates left it)
+        const T *D = ring + (d % STG) * psz, *Lp = D + 256;
+        if (tid == SW_THREADS - 1) load_next();
         if (tid < 64) {
             T a[RB];
-            quad_mv<T, 0, RB>(a, Lp + 16 * np, 16, tid >> 2, tid & 3, w, x + k0, np, rc);
-            if ((tid & 3) == 0 && (tid >> 2) < w)
+            quad_mv<T, 0, RB>(a, D, 16, quad_o(tid), quad_q(tid), 16, x + k0 * RB);
+            if (quad_q(tid) == 0)
 #pragma unroll
-                for (int r = 0; r < RB; r++) if (r < rc) xs[k0 + (tid >> 2) + r * np] = a[r];
+                for (int r = 0; r < RB; r++) xs[(k0 + quad_o(tid)) * RB + r] = a[r];
         }
         __syncthreads();
-        // the rows beyond the block: two lanes per row, eight columns each
-        const int ra = UPPER ? 0 : k0 + w, re = UPPER ? k0 : np;
-        for (int i0 = ra; i0 < re; i0 += SW_THREADS / 2) {
-            const int row = i0 + (tid >> 1), h = tid & 1;
+        // the rows beyond the block: two lanes per row, eight columns each (columns beyond the pivots are zero)
+        const int ra = UPPER ? 0 : k0 + w, rl = UPPER ? k0 : np - k0 - w;
+        for (int i0 = 0; i0 < rl; i0 += SW_THREADS / 2) {
+            const int ii = i0 + (tid & 15) + 16 * (tid >> 5), h = (tid >> 4) & 1, row = ii < rl ? ii : 0;
             T s[RB];
 #pragma unroll
             for (int r = 0; r < RB; r++) s[r] = VT<T>::zero();
-            if (row < re) {
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const int cc = 2 * c + h;
-                    if (cc < w) {
-                        const T l = Lp[cc * np + row];
+            for (int c = 0; c < 8; c++) {
+                const T l = Lp[(2 * c + h) * rl + row];
+                const T *xv = xs + (k0 + 2 * c + h) * RB;
 #pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rc) s[r] = madd<T>(s[r], l, xs[k0 + cc + r * np]);
-                    }
-                }
+                for (int r = 0; r < RB; r++) s[r] = madd<T>(s[r], l, xv[r]);
             }
 #pragma unroll
             for (int r = 0; r < RB; r++) {
-                s[r] = add(s[r], shfl_xor_v<T>(s[r], 1));
-                if (r < rc && row < re && h == 0) x[row + r * np] = sub(x[row + r * np], s[r]);
+                s[r] = add(s[r], shfl_xor_v<T>(s[r], 16));
+                if (ii < rl && h == 0) x[(ra + ii) * RB + r] = sub(x[(ra + ii) * RB + r], s[r]);
             }
         }
     }
-    cp_async_wait_n<0>();
+    pipe.done += nbk;
+    return !__syncthreads_or(!ok);
+}
+// the barriers of a pipe (ends with a barrier)
+template <int STG> __device__ __forceinline__ TriPipe tri_pipe(unsigned long long *bars)
+{
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < STG; k++) bar_init(bars + k, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     __syncthreads();
+    return TriPipe{bars, 0};
 }
 // shared memory of tri16 (x, xs and the ring), in elements
-static inline int64_t tri16_elems(int64_t np, int64_t rb, int stg) { return 2 * np * rb + stg * (16 * np + 256); }
+static inline int64_t tri16_elems(int64_t np, int64_t rb, int stg) { return 2 * tri_pad((int)np) * rb + stg * (16 * np + 256); }
 
 // L sweep of a level's small fronts, a CTA each (the successor of k_sv_fwdL): the front's vector in its final row order, x =
 // L11^-1 v (into Y in pivot order), then the contribution u = v[np:] - L21 x into VB, a thread per row with L's row read
 // once for all of the pass's right-hand sides
 template <typename T, int RB>
 __global__ void __launch_bounds__(SW_THREADS) k_sw_fwdL(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                        const T *__restrict__ La, const T *__restrict__ dinv,
+                                                        const T *__restrict__ La, const T *__restrict__ pk,
                                                         const int64_t *__restrict__ rowinit, const int *__restrict__ permall,
                                                         const int64_t *__restrict__ rsp, const int64_t *__restrict__ rsi,
                                                         const T *__restrict__ R, T *__restrict__ Y, T *__restrict__ VB, int64_t vstride,
-                                                        int64_t n, int nrhs)
+                                                        int64_t n, int nrhs, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SvFront F = fr[list[blockIdx.x]];
     const int nr = (int)F.nr, np = (int)(F.np < F.nr ? F.np : F.nr), nri = (int)F.nri, tid = threadIdx.x, m = nr - np;
-    T *x = reinterpret_cast<T *>(smem_raw), *xs = x + np * RB, *v = xs + np * RB, *ring = v + m * RB;     // v: the rows below the pivots
+    const int npd = tri_pad(np), psz = 16 * np + 256;
+    T *ring = reinterpret_cast<T *>(smem_raw), *x = ring + 2 * psz, *xs = x + npd * RB, *v = xs + npd * RB;       // v: the rows below the pivots, v[t + r * m]
+    __shared__ unsigned long long bars[2];
+    TriPipe pipe = tri_pipe<2>(bars);
+    for (int e = tid; e < npd * RB; e += SW_THREADS) x[e] = VT<T>::zero();
+    __syncthreads();
     const T *L = La + F.L_off;
     const int *perm = permall + F.row_off;
     pdl_wait();
@@ -108,11 +114,11 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_fwdL(const SvFront *__restric
             const int64_t g = F.row_off + i, ri = rowinit[g], q0 = rsp[g], q1 = rsp[g + 1];
             T val = (i < nri && ri >= 0) ? R[ri + (int64_t)(r0 + r) * n] : VT<T>::zero();
             for (int64_t q = q0; q < q1; q++) val = add(val, VB[rsi[q] + (int64_t)(r0 + r) * vstride]);
-            if (k < np) x[k + r * np] = val; else v[k - np + r * m] = val;
+            if (k < np) x[k * RB + r] = val; else v[k - np + r * m] = val;
         }
         __syncthreads();
-        tri16<T, false, RB, 2>(L, nr, np, x, xs, rc, dinv + F.d_off * 512, ring);
-        for (int e = tid; e < np * rc; e += SW_THREADS) Y[F.f + e % np + (int64_t)(r0 + e / np) * n] = xs[e];
+        if (!tri16<T, false, RB, 2>(pk + F.l_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+        for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; Y[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
         for (int t = tid; t < m; t += SW_THREADS) {
             T acc[RB];
 #pragma unroll
@@ -125,12 +131,14 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_fwdL(const SvFront *__restric
                 for (int q = 0; q < 16; q++)
                     if (k0 + q < np)
 #pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rc) acc[r] = madd<T>(acc[r], lv[q], xs[k0 + q + r * np]);
+                        for (int r = 0; r < RB; r++) acc[r] = madd<T>(acc[r], lv[q], xs[(k0 + q) * RB + r]);
             }
 #pragma unroll
             for (int r = 0; r < RB; r++)
                 if (r < rc) VB[F.row_off + np + t + (int64_t)(r0 + r) * vstride] = sub(v[t + r * m], acc[r]);
         }
+        __syncthreads();
+        if (r0 + RB < nrhs) for (int e = tid; e < npd * RB; e += SW_THREADS) x[e] = VT<T>::zero();
         __syncthreads();
     }
 }
@@ -141,16 +149,22 @@ static inline int64_t sw_fwdL_elems(int64_t nr, int64_t np, int64_t rb) { return
 // groups' sums added in order), then x = U11^-1 (y - the product)
 template <typename T, int RB>
 __global__ void __launch_bounds__(SW_THREADS) k_sw_bwdU(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                        const T *__restrict__ La, const T *__restrict__ Ua, const T *__restrict__ dinv,
+                                                        const T *__restrict__ La, const T *__restrict__ Ua, const T *__restrict__ pk,
                                                         const int64_t *__restrict__ cols, const T *__restrict__ Y, T *__restrict__ X,
-                                                        int64_t n, int nrhs)
+                                                        int64_t n, int nrhs, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SvFront F = fr[list[blockIdx.x]];
     const int np = (int)F.np, ncb = (int)(F.nc - F.np), tid = threadIdx.x;
     if (np == 0) { pdl_wait(); return; }
     const int G = SW_THREADS / np;                     // column groups (np <= 64)
-    T *x = reinterpret_cast<T *>(smem_raw), *xs = x + np * RB, *xc = xs + np * RB, *red = xc + ncb * RB, *ring = red + SW_THREADS * RB;
+    const int npd = tri_pad(np), psz = 16 * np + 256;
+    T *ring = reinterpret_cast<T *>(smem_raw), *x = ring + 2 * psz, *xs = x + npd * RB, *xc = xs + npd * RB, *red = xc + ncb * RB;
+    __shared__ unsigned long long bars[2];
+    TriPipe pipe = tri_pipe<2>(bars);
+    for (int e = tid; e < npd * RB; e += SW_THREADS) x[e] = VT<T>::zero();
+    for (int e = tid; e < ncb * RB; e += SW_THREADS) xc[e] = VT<T>::zero();
+    __syncthreads();
     const T *U12 = Ua + F.U_off;
     const int64_t *cb = cols + F.col_off + np;
     pdl_wait();
@@ -176,7 +190,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_bwdU(const SvFront *__restric
                 for (int q = 0; q < 8; q++)
                     if (t0 + q * G < ncb)
 #pragma unroll
-                        for (int r = 0; r < RB; r++) if (r < rc) acc[r] = madd<T>(acc[r], u[q], xc[(t0 + q * G) * RB + r]);
+                        for (int r = 0; r < RB; r++) acc[r] = madd<T>(acc[r], u[q], xc[(t0 + q * G) * RB + r]);
             }
 #pragma unroll
             for (int r = 0; r < RB; r++) red[(g * RB + r) * np + i] = acc[r];
@@ -186,11 +200,11 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_bwdU(const SvFront *__restric
             const int ii = e % np, r = e / np;
             T s = VT<T>::zero();
             for (int gg = 0; gg < G; gg++) s = add(s, red[(gg * RB + r) * np + ii]);
-            x[e] = sub(Y[F.f + ii + (int64_t)(r0 + r) * n], s);
+            x[ii * RB + r] = sub(Y[F.f + ii + (int64_t)(r0 + r) * n], s);
         }
         __syncthreads();
-        tri16<T, true, RB, 2>(La + F.L_off, F.nr, np, x, xs, rc, dinv + F.d_off * 512, ring);
-        for (int e = tid; e < np * rc; e += SW_THREADS) X[F.f + e % np + (int64_t)(r0 + e / np) * n] = xs[e];
+        if (!tri16<T, true, RB, 2>(pk + F.u_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+        for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; X[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
         __syncthreads();
     }
 }
@@ -200,21 +214,27 @@ static inline int64_t sw_bwdU_elems(int64_t nc, int64_t np, int64_t rb) { return
 // VB in place and into Y in pivot order
 template <typename T, int RB, int STG>
 __global__ void __launch_bounds__(SW_THREADS) k_swb_L11(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                        const T *__restrict__ La, const T *__restrict__ dinv, T *__restrict__ VB,
-                                                        int64_t vstride, T *__restrict__ Y, int64_t n, int nrhs)
+                                                        const T *__restrict__ pk, T *__restrict__ VB,
+                                                        int64_t vstride, T *__restrict__ Y, int64_t n, int nrhs, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SvFront F = fr[list[blockIdx.x]];
     const int np = (int)(F.np < F.nr ? F.np : F.nr), tid = threadIdx.x, r0 = blockIdx.y * RB, rc = nrhs - r0 < RB ? nrhs - r0 : RB;
     if (np == 0) return;
-    T *x = reinterpret_cast<T *>(smem_raw), *xs = x + np * RB, *ring = xs + np * RB;
-    for (int e = tid; e < np * rc; e += SW_THREADS) x[e] = VB[F.row_off + e % np + (int64_t)(r0 + e / np) * vstride];
+    const int npd = tri_pad(np), psz = 16 * np + 256;
+    T *ring = reinterpret_cast<T *>(smem_raw), *x = ring + STG * psz, *xs = x + npd * RB;
+    __shared__ unsigned long long bars[STG];
+    TriPipe pipe = tri_pipe<STG>(bars);
+    for (int e = tid; e < npd * RB; e += SW_THREADS) {
+        const int k = e % npd, r = e / npd;
+        x[k * RB + r] = k < np && r < rc ? VB[F.row_off + k + (int64_t)(r0 + r) * vstride] : VT<T>::zero();
+    }
     __syncthreads();
-    tri16<T, false, RB, STG>(La + F.L_off, F.nr, np, x, xs, rc, dinv + F.d_off * 512, ring);
+    if (!tri16<T, false, RB, STG>(pk + F.l_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
     for (int e = tid; e < np * rc; e += SW_THREADS) {
-        const int k = e % np, r = r0 + e / np;
-        VB[F.row_off + k + (int64_t)r * vstride] = xs[e];
-        Y[F.f + k + (int64_t)r * n] = xs[e];
+        const int k = e % np, r = e / np;
+        VB[F.row_off + k + (int64_t)(r0 + r) * vstride] = xs[k * RB + r];
+        Y[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r];
     }
 }
 
@@ -234,7 +254,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_L21(const SvFront *__restric
     const bool on = row < F.nr;
     for (int r0 = 0; r0 < nrhs; r0 += RB) {
         const int rc = nrhs - r0 < RB ? nrhs - r0 : RB;
-        for (int e = tid; e < np * rc; e += SW_THREADS) xs[(e % np) * RB + e / np] = VB[F.row_off + e % np + (int64_t)(r0 + e / np) * vstride];
+        for (int e = tid; e < np * RB; e += SW_THREADS) { const int k = e % np, r = e / np; xs[k * RB + r] = r < rc ? VB[F.row_off + k + (int64_t)(r0 + r) * vstride] : VT<T>::zero(); }
         __syncthreads();
         T acc[RB];
 #pragma unroll
@@ -247,7 +267,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_L21(const SvFront *__restric
             for (int q = 0; q < 16; q++)
                 if (k0 + 8 * q < np)
 #pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rc) acc[r] = madd<T>(acc[r], lv[q], xs[(k0 + 8 * q) * RB + r]);
+                    for (int r = 0; r < RB; r++) acc[r] = madd<T>(acc[r], lv[q], xs[(k0 + 8 * q) * RB + r]);
         }
 #pragma unroll
         for (int r = 0; r < RB; r++) red[(g * RB + r) * 32 + rl] = acc[r];
@@ -288,7 +308,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_u12(const SvFront *__restric
         for (int k = tid; k < cc; k += SW_THREADS) {
             const T *xr = X + cb[k] + (int64_t)r0 * n;
 #pragma unroll
-            for (int r = 0; r < RB; r++) if (r < rc) Xs[k * RB + r] = xr[(int64_t)r * n];
+            for (int r = 0; r < RB; r++) Xs[k * RB + r] = r < rc ? xr[(int64_t)r * n] : VT<T>::zero();
         }
         __syncthreads();
         T acc[RB];
@@ -302,7 +322,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_u12(const SvFront *__restric
             for (int q = 0; q < 16; q++)
                 if (k0 + 4 * q < cc)
 #pragma unroll
-                    for (int r = 0; r < RB; r++) if (r < rc) acc[r] = madd<T>(acc[r], u[q], Xs[(k0 + 4 * q) * RB + r]);
+                    for (int r = 0; r < RB; r++) acc[r] = madd<T>(acc[r], u[q], Xs[(k0 + 4 * q) * RB + r]);
         }
 #pragma unroll
         for (int r = 0; r < RB; r++) red[(g * RB + r) * 64 + rl] = acc[r];
@@ -320,74 +340,40 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_u12(const SvFront *__restric
 // (blockIdx.y); presummed: k_svb_psum left y - the products in the front's first partial sum
 template <typename T, int RB, int STG>
 __global__ void __launch_bounds__(SW_THREADS) k_swb_bwdU(const SvFront *__restrict__ fr, const int *__restrict__ list,
-                                                         const T *__restrict__ La, const T *__restrict__ dinv, const T *__restrict__ part,
-                                                         const T *__restrict__ Y, T *__restrict__ X, int64_t n, int nrhs, int presummed)
+                                                         const T *__restrict__ pk, const T *__restrict__ part,
+                                                         const T *__restrict__ Y, T *__restrict__ X, int64_t n, int nrhs, int presummed, DevStatus *st)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const SvFront F = fr[list[blockIdx.x]];
     const int np = (int)F.np, tid = threadIdx.x, r0 = blockIdx.y * RB, rc = nrhs - r0 < RB ? nrhs - r0 : RB;
     if (np == 0) return;
-    T *x = reinterpret_cast<T *>(smem_raw), *xs = x + np * RB, *ring = xs + np * RB;
+    const int npd = tri_pad(np), psz = 16 * np + 256;
+    T *ring = reinterpret_cast<T *>(smem_raw), *x = ring + STG * psz, *xs = x + npd * RB;
     const T *pp = part + F.poff * nrhs;
-    for (int e = tid; e < np * rc; e += SW_THREADS) {
-        const int i = e % np;
-        const int64_t r = r0 + e / np;
-        T v;
-        if (presummed && F.nch > 0) v = pp[i + r * np];
-        else {
-            v = Y[F.f + i + r * n];
-            for (int64_t q0 = 0; q0 < F.nch; q0 += 16) {     // sixteen loads in flight, the sum in chunk order
-                T pv[16];
+    __shared__ unsigned long long bars[STG];
+    TriPipe pipe = tri_pipe<STG>(bars);
+    for (int e = tid; e < npd * RB; e += SW_THREADS) {
+        const int i = e % npd, rr = e / npd;
+        const int64_t r = r0 + rr;
+        T v = VT<T>::zero();
+        if (i < np && rr < rc) {
+            if (presummed && F.nch > 0) v = pp[i + r * np];
+            else {
+                v = Y[F.f + i + r * n];
+                for (int64_t q0 = 0; q0 < F.nch; q0 += 16) {     // sixteen loads in flight, the sum in chunk order
+                    T pv[16];
 #pragma unroll
-                for (int q = 0; q < 16; q++) pv[q] = q0 + q < F.nch ? pp[(q0 + q) * np * nrhs + i + r * np] : VT<T>::zero();
+                    for (int q = 0; q < 16; q++) pv[q] = q0 + q < F.nch ? pp[(q0 + q) * np * nrhs + i + r * np] : VT<T>::zero();
 #pragma unroll
-                for (int q = 0; q < 16; q++) if (q0 + q < F.nch) v = sub(v, pv[q]);
+                    for (int q = 0; q < 16; q++) if (q0 + q < F.nch) v = sub(v, pv[q]);
+                }
             }
         }
-        x[e] = v;
+        x[i * RB + rr] = v;
     }
     __syncthreads();
-    tri16<T, true, RB, STG>(La + F.L_off, F.nr, np, x, xs, rc, dinv + F.d_off * 512, ring);
-    for (int e = tid; e < np * rc; e += SW_THREADS) X[F.f + e % np + (int64_t)(r0 + e / np) * n] = xs[e];
-}
-
-// The inverses of the 16 x 16 diagonal blocks of every front's U11 and unit-lower L11: block b of a front at
-// dinv[(d_off + b) * 512] (U's, then L's 256 later), column-major, identity beyond the front's pivots; a thread per column,
-// four blocks per CTA.  (A zero diagonal of U cannot be met: the factorization reports the column as singular.)
-template <typename T>
-__global__ void __launch_bounds__(128) k_front_dinv(const SvFront *__restrict__ fr, const int *__restrict__ dfront, int64_t nblk,
-                                                    const T *__restrict__ La, T *__restrict__ dinv, const DevStatus *st)
-{
-    if (st->code) return;
-    const int64_t blk = blockIdx.x * (int64_t)4 + (threadIdx.x >> 5);
-    if (blk >= nblk) return;
-    const SvFront F = fr[dfront[blk]];
-    const int lower = (threadIdx.x >> 4) & 1, c = threadIdx.x & 15;
-    const int np = (int)(F.np < F.nr ? F.np : F.nr), k0 = 16 * (int)(blk - F.d_off);
-    const T *L = La + F.L_off;
-    T x[16];
-    auto at = [&](int i, int k) -> T { return k0 + i < np && k0 + k < np ? L[(k0 + i) + (int64_t)(k0 + k) * F.nr] : VT<T>::zero(); };
-    if (lower) {
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            T s = i == c ? VT<T>::one() : VT<T>::zero();
-#pragma unroll
-            for (int k = 0; k < i; k++) s = msub(s, at(i, k), x[k]);
-            x[i] = s;
-        }
-    } else {
-#pragma unroll
-        for (int i = 15; i >= 0; i--) {
-            T s = i == c ? VT<T>::one() : VT<T>::zero();
-#pragma unroll
-            for (int k = 15; k > i; k--) s = msub(s, at(i, k), x[k]);
-            const T d = at(i, i);
-            x[i] = k0 + i < np ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
-        }
-    }
-    T *o = dinv + blk * 512 + 256 * lower + c * 16;
-#pragma unroll
-    for (int i = 0; i < 16; i++) o[i] = x[i];
+    if (!tri16<T, true, RB, STG>(pk + F.u_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+    for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; X[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
 }
 
 }  // namespace fpl
