@@ -73,43 +73,50 @@ __global__ void k_scale_raw(double *d, int64_t m, double sc)
 __device__ __forceinline__ double sqmod(double a) { return __dmul_rn(a, a); }
 __device__ __forceinline__ double sqmod(cplx a) { return __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)); }
 
-// row maxima of |b|^2 (order independent: the maximum of non-negative doubles is their integer maximum)
+// The iterations run as four launches each (row scale, column pass, column scale, column apply) with no host decision: res[it]
+// takes iteration it's residual, and a launch of iteration it does nothing once res[it - 1] is below tol (an iteration
+// that did nothing leaves its residual at zero).  A zero row or column stops them through the status word.  (Four launches
+// instead of nine, and one residual atomic per warp instead of per row: the row and column scales of n = 160,801 took
+// 28 us each, 160,801 atomics on one word.)
+__device__ __forceinline__ bool ruiz_idle(const unsigned long long *res, int it, double tol) { return it > 0 && bitsd(res[it - 1]) < tol; }
+
+// row maxima of |b|^2 before the first iteration (order independent: the maximum of non-negative doubles is their integer
+// maximum); the later iterations' come from the column apply
 template <typename T>
 __global__ void k_ruiz_rowmax(const int64_t *__restrict__ Bi, const T *__restrict__ Bx, int64_t nnz,
                               unsigned long long *__restrict__ rmax, const DevStatus *st)
 {
-    if (st->done || st->code) return;
+    if (st->code) return;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x)
         atomicMax(&rmax[Bi[p]], dbits(sqmod(Bx[p])));
 }
 
 // zero-row check, residual, row scale 1/sqrt(sqrt(max)), Dr *= scale (FPLUS src/equil.c:80-92); the column maxima of
-// the coming column pass start at zero
-__global__ void k_ruiz_rowscale(int64_t n, unsigned long long *__restrict__ rmax, double *__restrict__ Dr,
-                                unsigned long long *__restrict__ cmax, DevStatus *st)
+// the coming column pass start at zero.  Columns likewise (FPLUS src/equil.c:148-155; the row maxima of the coming column
+// apply start at zero).  zero_code: what a zero line reports, the smallest index winning (the reference reports the first);
+// a launch goes on past lines that this launch itself has reported, so that the smallest does not depend on the order
+__global__ void k_ruiz_scale(int64_t n, unsigned long long *__restrict__ mx, double *__restrict__ D, unsigned long long *__restrict__ next,
+                             int zero_code, unsigned long long *__restrict__ res, int it, double tol, DevStatus *st)
 {
-    if (st->done || st->code) return;
+    if (ruiz_idle(res, it, tol)) return;
+    const int code = *(volatile int *)&st->code;
+    if (code != 0 && code != zero_code) return;
+    double worst = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        cmax[i] = 0ull;
-        double m = bitsd(rmax[i]);
-        if (m == 0.0) {           // the smallest zero row wins (the reference reports the first)
-            atomicCAS(&((DevStatus *)st)->code, 0, ST_ZERO_ROW);
+        next[i] = 0ull;
+        const double m = bitsd(mx[i]);
+        if (m == 0.0) {
+            atomicCAS(&st->code, 0, zero_code);
+            atomicMin((unsigned long long *)&st->idx, (unsigned long long)i);
             continue;
         }
-        double v = 0.5 * fabs(log(m));
-        atomicMax(&st->res_bits, dbits(v));
-        double dr = 1.0 / sqrt(sqrt(m));
-        Dr[i] = __dmul_rn(Dr[i], dr);
-        rmax[i] = dbits(dr);
+        worst = fmax(worst, 0.5 * fabs(log(m)));
+        const double d = 1.0 / sqrt(sqrt(m));
+        D[i] = __dmul_rn(D[i], d);
+        mx[i] = dbits(d);
     }
-}
-
-// zero-row index: the smallest (second pass so the index is deterministic)
-__global__ void k_first_zero(int64_t n, const unsigned long long *__restrict__ v, DevStatus *st, int code)
-{
-    if (st->code != code || st->done) return;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        if (bitsd(v[i]) == 0.0) atomicMin((unsigned long long *)&st->idx, (unsigned long long)i);
+    const unsigned long long w = warp_max_key(dbits(worst));
+    if ((threadIdx.x & 31) == 0 && w != 0ull) atomicMax(&res[it], w);
 }
 
 // Column passes run over column segments of at most COL_SEG entries (seg: column, first entry, end; a warp each), so a
@@ -121,9 +128,9 @@ constexpr int64_t COL_SEG = 1024;
 template <typename T>
 __global__ void k_ruiz_colpass(const int64_t *__restrict__ seg, int64_t nseg, const int64_t *__restrict__ Bi, T *__restrict__ Bx,
                                const unsigned long long *__restrict__ rscale, unsigned long long *__restrict__ cmax,
-                               const DevStatus *st)
+                               const unsigned long long *__restrict__ res, int it, double tol, const DevStatus *st)
 {
-    if (st->done || st->code) return;
+    if (ruiz_idle(res, it, tol) || st->code) return;
     const int lane = threadIdx.x & 31;
     for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; g < nseg; g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const int64_t j = seg[3 * g], p1 = seg[3 * g + 2];
@@ -138,42 +145,31 @@ __global__ void k_ruiz_colpass(const int64_t *__restrict__ seg, int64_t nseg, co
     }
 }
 
-// the zero-column check, residual, column scale, Dc *= scale (FPLUS src/equil.c:148-155)
-__global__ void k_ruiz_colscale(int64_t n, unsigned long long *__restrict__ cmax, double *__restrict__ Dc, DevStatus *st)
-{
-    if (st->done || st->code) return;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-        double m = bitsd(cmax[j]);
-        if (m == 0.0) { atomicCAS(&st->code, 0, ST_ZERO_COL); continue; }
-        double v = 0.5 * fabs(log(m));
-        atomicMax(&st->res_bits, dbits(v));
-        double c = 1.0 / sqrt(sqrt(m));
-        Dc[j] = __dmul_rn(Dc[j], c);
-        cmax[j] = dbits(c);
-    }
-}
-
+// scale by the column scales; and the row maxima of |b|^2 for the next iteration (rmax null: none)
 template <typename T>
-__global__ void k_ruiz_colapply(const int64_t *__restrict__ seg, int64_t nseg, T *__restrict__ Bx,
-                                const unsigned long long *__restrict__ cscale, const DevStatus *st)
+__global__ void k_ruiz_colapply(const int64_t *__restrict__ seg, int64_t nseg, const int64_t *__restrict__ Bi, T *__restrict__ Bx,
+                                const unsigned long long *__restrict__ cscale, unsigned long long *__restrict__ rmax,
+                                const unsigned long long *__restrict__ res, int it, double tol, const DevStatus *st)
 {
-    if (st->done || st->code) return;
+    if (ruiz_idle(res, it, tol) || st->code) return;
     const int lane = threadIdx.x & 31;
     for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; g < nseg; g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const double c = bitsd(cscale[seg[3 * g]]);
         const int64_t p1 = seg[3 * g + 2];
-        for (int64_t p = seg[3 * g + 1] + lane; p < p1; p += 32) Bx[p] = scal(Bx[p], c);
+        for (int64_t p = seg[3 * g + 1] + lane; p < p1; p += 32) {
+            const T v = scal(Bx[p], c);
+            Bx[p] = v;
+            if (rmax) atomicMax(&rmax[Bi[p]], dbits(sqmod(v)));
+        }
     }
 }
 
-// end of an iteration: count it, stop when the residual is below tol (FPLUS src/equil.c:405-411)
-__global__ void k_ruiz_check(DevStatus *st, double tol)
+// the iterations that ran: up to the first whose residual is below tol (FPLUS src/equil.c:405-411)
+__global__ void k_ruiz_count(const unsigned long long *res, int max_iter, double tol, DevStatus *st)
 {
-    if (st->done) return;
-    if (st->code) { st->done = 1; return; }      // an error: later iterations change nothing (the index stays)
-    st->iters++;
-    if (bitsd(st->res_bits) < tol) st->done = 1;
-    st->res_bits = 0ull;
+    int k = 0;
+    while (k < max_iter && !ruiz_idle(res, k, tol)) k++;
+    st->iters = k;
 }
 
 __global__ void k_fold(double *Dr, double *Dc, int64_t n, double h)

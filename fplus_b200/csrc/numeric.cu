@@ -387,7 +387,7 @@ DevNum::~DevNum()
     if (device >= 0) cudaSetDevice(device);
     for (void *p : {(void *)Ax, (void *)Bx, (void *)Drp, (void *)Dcp, (void *)colmax, (void *)Larena, (void *)Uarena,
                     (void *)cbstack, (void *)work, (void *)rowid, (void *)p_lu, (void *)pinv, (void *)ipiv, (void *)perm,
-                    (void *)st, (void *)scratch, (void *)rbuf, (void *)sbuf, (void *)xbuf, (void *)part, (void *)work2,
+                    (void *)st, (void *)scratch, (void *)rzres, (void *)rbuf, (void *)sbuf, (void *)xbuf, (void *)part, (void *)work2,
                     (void *)perm2, (void *)rr_p, (void *)rr_l, (void *)rr_s, (void *)ir_b, (void *)ir_x, (void *)ir_r,
                     (void *)ir_d, (void *)ir_bits, scratch_norm, tcws, gm_buf, coopbuf, (void *)permall, vbuf, bsw, bscb, pk, (void *)chsync, chacc})
         if (p) cudaFreeAsync(p, stream);
@@ -476,6 +476,25 @@ static int run_equil(const DevPlan &D, DevNum &N, int equilibrate, int max_iter,
     cudaStream_t s = N.stream;
     const int64_t n = N.n, nnz = N.nnz;
     T *Bx = (T *)N.Bx;
+    // the Ruiz iterations (four launches each; they do nothing once converged)
+    auto ruiz = [&]() -> int {
+        if (max_iter <= 0) return FPLUS_OK;
+        unsigned long long *rmax = (unsigned long long *)N.scratch, *cmax = rmax + n;
+        int rc;
+        if ((rc = ensure_async(N, (void **)&N.rzres, &N.cap_rz, (size_t)(max_iter + 1) * 8, err, errlen))) return rc;
+        CK(cudaMemsetAsync(N.rzres, 0, (size_t)(max_iter + 1) * 8, s));
+        CK(cudaMemsetAsync(rmax, 0, (size_t)n * 8, s));
+        k_ruiz_rowmax<T><<<nblk(nnz), 256, 0, s>>>(D.Bi, Bx, nnz, rmax, N.st), note_launch();
+        for (int it = 0; it < max_iter; it++) {
+            k_ruiz_scale<<<nblk(n), 256, 0, s>>>(n, rmax, N.Drp, cmax, ST_ZERO_ROW, N.rzres, it, tol, N.st), note_launch();
+            k_ruiz_colpass<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, D.Bi, Bx, rmax, cmax, N.rzres, it, tol, N.st), note_launch();
+            k_ruiz_scale<<<nblk(n), 256, 0, s>>>(n, cmax, N.Dcp, rmax, ST_ZERO_COL, N.rzres, it, tol, N.st), note_launch();
+            k_ruiz_colapply<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, D.Bi, Bx, cmax, it + 1 < max_iter ? rmax : nullptr, N.rzres, it,
+                                                                tol, N.st), note_launch();
+        }
+        k_ruiz_count<<<1, 1, 0, s>>>(N.rzres, max_iter, tol, N.st), note_launch();
+        return FPLUS_OK;
+    };
     k_gather<T><<<nblk(nnz), 256, 0, s>>>(Bx, (const T *)N.Ax, D.Bsrc, nnz), note_launch();
     if (N.capture) {
         // the same steps without host copies or decisions: the set-up on the device, every Ruiz iteration launched (the
@@ -487,18 +506,8 @@ static int run_equil(const DevPlan &D, DevNum &N, int equilibrate, int max_iter,
             const int64_t m = (N.cplx ? 2 : 1) * nnz;
             k_abs_range<<<nblk(m), 256, 0, s>>>((const double *)Bx, m, N.st), note_launch();
             k_range_flag<<<1, 1, 0, s>>>(N.st), note_launch();
-            unsigned long long *rmax = (unsigned long long *)N.scratch, *cmax = rmax + n;
-            for (int it = 0; it < max_iter; it++) {
-                CK(cudaMemsetAsync(rmax, 0, (size_t)n * 8, s));
-                k_ruiz_rowmax<T><<<nblk(nnz), 256, 0, s>>>(D.Bi, Bx, nnz, rmax, N.st), note_launch();
-                k_ruiz_rowscale<<<nblk(n), 256, 0, s>>>(n, rmax, N.Drp, cmax, N.st), note_launch();
-                k_first_zero<<<nblk(n), 256, 0, s>>>(n, rmax, N.st, ST_ZERO_ROW), note_launch();
-                k_ruiz_colpass<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, D.Bi, Bx, rmax, cmax, N.st), note_launch();
-                k_ruiz_colscale<<<nblk(n), 256, 0, s>>>(n, cmax, N.Dcp, N.st), note_launch();
-                k_first_zero<<<nblk(n), 256, 0, s>>>(n, cmax, N.st, ST_ZERO_COL), note_launch();
-                k_ruiz_colapply<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, Bx, cmax, N.st), note_launch();
-                k_ruiz_check<<<1, 1, 0, s>>>(N.st, tol), note_launch();
-            }
+            int rrc;
+            if ((rrc = ruiz())) return rrc;
         }
         CK(cudaMemsetAsync(N.colmax, 0, (size_t)n * 8, s));
         k_colmax<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, Bx, (unsigned long long *)N.colmax), note_launch();
@@ -543,18 +552,8 @@ static int run_equil(const DevPlan &D, DevNum &N, int equilibrate, int max_iter,
             k4 = -((emax + emin) / 2 / 4) * 4;
             k_scale_raw<<<nblk(m), 256, 0, s>>>((double *)Bx, m, std::ldexp(1.0, k4)), note_launch();
         }
-        unsigned long long *rmax = (unsigned long long *)N.scratch, *cmax = rmax + n;
-        for (int it = 0; it < max_iter; it++) {
-            CK(cudaMemsetAsync(rmax, 0, (size_t)n * 8, s));
-            k_ruiz_rowmax<T><<<nblk(nnz), 256, 0, s>>>(D.Bi, Bx, nnz, rmax, N.st), note_launch();
-            k_ruiz_rowscale<<<nblk(n), 256, 0, s>>>(n, rmax, N.Drp, cmax, N.st), note_launch();
-            k_first_zero<<<nblk(n), 256, 0, s>>>(n, rmax, N.st, ST_ZERO_ROW), note_launch();
-            k_ruiz_colpass<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, D.Bi, Bx, rmax, cmax, N.st), note_launch();
-            k_ruiz_colscale<<<nblk(n), 256, 0, s>>>(n, cmax, N.Dcp, N.st), note_launch();
-            k_first_zero<<<nblk(n), 256, 0, s>>>(n, cmax, N.st, ST_ZERO_COL), note_launch();
-            k_ruiz_colapply<T><<<nblk(32 * D.nseg), 256, 0, s>>>(D.seg, D.nseg, Bx, cmax, N.st), note_launch();
-            k_ruiz_check<<<1, 1, 0, s>>>(N.st, tol), note_launch();
-        }
+        int rrc;
+        if ((rrc = ruiz())) return rrc;
         if (k4 != 0) k_fold<<<nblk(n), 256, 0, s>>>(N.Drp, N.Dcp, n, std::ldexp(1.0, k4 / 2)), note_launch();
     }
     CK(cudaMemsetAsync(N.colmax, 0, (size_t)n * 8, s));

@@ -111,6 +111,8 @@ struct DevNum {
     cudaEvent_t ev_lu = nullptr, ev_head = nullptr;
     DevStatus *st = nullptr;
     void *scratch = nullptr;
+    unsigned long long *rzres = nullptr;     // the Ruiz iterations' residuals
+    size_t cap_rz = 0;
     void *scratch_norm = nullptr;
     size_t cap_norm = 0;
     // the precision form: the arithmetic of the large fronts' Schur updates (schur_tc.hpp), their operand workspace, and
