@@ -620,15 +620,15 @@ __global__ void __launch_bounds__(1024) k_mc_order(int nrows, int npr, const int
 }
 
 // the pivot block in the final row order into the arena: row k of L \ U takes W's row perm[k], except the pivot rows'
-// entries right of their own panel, which are U12 (Ub)
+// entries right of their own panel (pw columns), which are U12 (Ub)
 template <typename T>
-__global__ void k_mc_lout(const T *__restrict__ W, int64_t ld, int64_t nrows, int64_t npiv, int64_t npr,
+__global__ void k_mc_lout(const T *__restrict__ W, int64_t ld, int64_t nrows, int64_t npiv, int64_t npr, int pw,
                           const int *__restrict__ perm, const T *__restrict__ Ub, T *__restrict__ Lout, const DevStatus *st)
 {
     if (st->code) return;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nrows * npiv; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t k = e % nrows, c = e / nrows;
-        const int64_t pend = k < npr ? ((k / MC_PW + 1) * MC_PW < npr ? (k / MC_PW + 1) * MC_PW : npr) : 0;
+        const int64_t pend = k < npr ? ((k / pw + 1) * pw < npr ? (k / pw + 1) * pw : npr) : 0;
         Lout[e] = (k < npr && c >= pend) ? Ub[k + c * npiv] : W[perm[k] + c * ld];
     }
 }

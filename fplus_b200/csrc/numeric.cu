@@ -842,7 +842,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             bool done = false;
             if (any_mc && !(N.lu_variant & 4)) {
                 // (the cluster form as far as its CTAs hold the rows, with as many CTAs as the cluster takes; above, the
-                // grid form over the SMs: a step of it costs about 4 us, a global round trip, against 0.6 us)
+                // grid form over the SMs: a step of it costs about 4 us, a global round trip, against 1.2 us real, 2 us complex)
                 const bool cl = mc_cl > 0 && nr <= (int64_t)mc_cl * per_max;
                 int G = cl ? (int)std::min<int64_t>(mc_cl, std::max<int64_t>(2, (nr + 31) / 32))
                            : (int)std::min<int64_t>(mc_sms, std::max<int64_t>(1, (nr + 63) / 64));
@@ -878,7 +878,7 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
                     note_launch();
                     k_mc_order<T><<<1, 1024, 0, st>>>((int)nr, (int)npr, mc_chosen, N.rowid + F.row_off, perm, F.f, N.p_lu,
                                                       mc_markp, mc_ridp, N.st), note_launch();
-                    k_mc_lout<T><<<nblk(nr * np), 256, 0, st>>>(W, ld, nr, np, npr, perm, mc_U, Lf, N.st), note_launch();
+                    k_mc_lout<T><<<nblk(nr * np), 256, 0, st>>>(W, ld, nr, np, npr, cl && G <= mc_cl ? cl_pw<T>() : MC_PW, perm, mc_U, Lf, N.st), note_launch();
                     done = true;
                 } else (void)cudaGetLastError();
             }

@@ -1,8 +1,9 @@
 """The panel pivot-block LU (k_front_lu6) at the sizes where it can go wrong: dense matrices in the identity orders, so that
 one front (or a few) holds the whole matrix: fewer pivots than a panel, the last panel partial, full and alone, rows at the
 edges of a warp and of the 128-row form, blocks over 128 rows; equal moduli in a column, moduli whose squares leave the
-range, a singular column, and the shared-memory form (variant 1) on the same blocks.  The bar is that of the parity tests:
-the oracle's pivots, L and U within 1e-12."""
+range, a singular column, and the shared-memory form (variant 1) on the same blocks.  Then the cluster form (k_block_lu_cl)
+on larger ones: rows and panels that do not divide, the shortest and longest shares of a CTA, the same special values, a
+tie between rows of different CTAs.  The bar is that of the parity tests: the oracle's pivots, L and U within 1e-12."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -73,6 +74,33 @@ def test_singular_column(gpu, cplx):
     n, Ap, Ai, Ax = _dense(40, cplx, 3)
     A = Ax.reshape(n, n)                       # row j: column j
     A[20] = A[3]                               # column 20 equals column 3
+    S = F.analyze(n, Ap, Ai, pin_dense=0, equilibrate=0)
+    with pytest.raises(F.FplusError) as e:
+        S.factor(Ax, F.default_options(equilibrate=0, pin_dense=0))
+    assert e.value.code == F.FPLUS_ERR_SINGULAR
+
+
+# (pivot blocks of n rows and up to 256 columns; per CTA n / 16 rows: 10 to 63, a share that ends in a partial warp; widths
+# that leave panels of 1, 15, 16, 17 and 31 columns)
+@pytest.mark.parametrize("n", [161, 175, 193, 224, 239, 255, 257, 272, 303, 513, 1000])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_cluster_sizes(gpu, cplx, n):
+    _check(_dense(n, cplx, n))
+
+
+@pytest.mark.parametrize("kind", ["ties", "tiny", "zeros"])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_cluster_values(gpu, cplx, kind):
+    _check(_dense(300, cplx, 7, kind), equilibrate=0 if kind != "zeros" else 1)
+
+
+@pytest.mark.parametrize("col", [1, 37, 250])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_cluster_singular_column(gpu, cplx, col):
+    """As above in a block of the cluster form: reported, at any step of a panel, by a kernel that ends."""
+    n, Ap, Ai, Ax = _dense(300, cplx, 3)
+    A = Ax.reshape(n, n)
+    A[col] = A[0]
     S = F.analyze(n, Ap, Ai, pin_dense=0, equilibrate=0)
     with pytest.raises(F.FplusError) as e:
         S.factor(Ax, F.default_options(equilibrate=0, pin_dense=0))
