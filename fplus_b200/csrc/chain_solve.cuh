@@ -9,7 +9,7 @@
 //              these appear, two or more blocks ahead of the solver (which takes the product with the block just solved
 //              itself, from shared memory).  U12's 64 x 64 blocks are contiguous and stream through a ring of shared
 //              memory without waiting for x.  Cross-CTA order: a counter of the blocks solved and a flag per block whose
-//              products are all in, release / acquire, waits bounded.  All CTAs are resident together: one cluster, or a
+//              products are all in, release / acquire, waits bounded.  All CTAs are resident together: a
 //              cooperative launch.
 //   k_chain_l  L (TR 0) or L^T (TR 1, 2) by one CTA per group of right-hand sides, the front's row vector in shared
 //              memory from front to front (no global round trip), L streamed in 16-column pieces.

@@ -681,6 +681,12 @@ __global__ void __launch_bounds__(128) k_trsm_unit(T *__restrict__ W, int64_t ld
 // Cout <- Cin - A B (column-major; M x K times K x N; Cin's rows optionally gathered through rmap) on the FP64 tensor cores: mma.sync m8n8k4 f64 (DMMA).  64 x 64 block
 // tiles, 16-deep K slices staged in shared memory, 8 warps of 32 x 16.  Complex: four real products per complex one
 // (Cr += Ar Br - Ai Bi, Ci += Ar Bi + Ai Br), the minus folded into a negated copy of Bi.
+// What bounds it (B200): the FP64 mma rate (about 33 TFLOP/s at 1.8 GHz) for large products; below about 150 tiles one
+// tile's own latency.  The epilogue's loads go out in batches: one at a time, each held back by the store before it (Cout
+// may be Cin), they were a third of a tile at K = 64.  Two CTAs an SM also for complex (138 -> 128 registers, a few spills)
+// so that one's products cover the other's staging.  Real, K = 256: 2,400^2 131.8 -> 118.9 us (24.8 TFLOP/s), 600^2 18.7 ->
+// 16.7; K = 64: 2,400^2 65.0 -> 45.4.  Complex, K = 256: 2,400^2 535.8 -> 428.6 us (27.5 TFLOP/s), 1,200^2 142.4 -> 137.5,
+// 600^2 49.5 -> 52.5 (one tile an SM: the spills).
 __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -690,7 +696,7 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 constexpr int GBM = 64, GBN = 64, GBK = 16, GPAD = 68, GBP = 20;   // A staged [k][m] (row 68), B staged [n][k] (row 20)
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_gemm_sub(int64_t M, int64_t N, int64_t K, const T *__restrict__ A, int64_t lda,
+__global__ void __launch_bounds__(256, 2) k_gemm_sub(int64_t M, int64_t N, int64_t K, const T *__restrict__ A, int64_t lda,
                                                  const T *__restrict__ B, int64_t ldb, const T *Cin, int64_t ldci,
                                                  const int *__restrict__ rmap, T *Cout, int64_t ldco, const DevStatus *st,
                                                  OutMap om)
@@ -772,26 +778,41 @@ __global__ void __launch_bounds__(256) k_gemm_sub(int64_t M, int64_t N, int64_t 
         }
         __syncthreads();
     }
+    // (Cout may be Cin: all loads of a batch are issued before its first store, which would otherwise hold them back)
+    constexpr int AB = CP ? 2 : 4;                       // 8-row fragments per batch
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a0 = 0; a0 < 4; a0 += AB) {
+        T v[AB][2][2];
 #pragma unroll
-        for (int b = 0; b < 2; b++)
+        for (int a = 0; a < AB; a++) {
+            const int64_t gm = m0 + wm * 32 + (a0 + a) * 8 + (lane >> 2);
+            const int64_t gi = rmap && gm < M ? (int64_t)rmap[gm] : gm;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int64_t gm = m0 + wm * 32 + a * 8 + (lane >> 2);
-                const int64_t gn = n0 + wn * 16 + b * 8 + 2 * (lane & 3) + h;
-                if (gm < M && gn < N) {
-                    const int64_t gi = rmap ? (int64_t)rmap[gm] : gm;
-                    T v = Cin[gi + gn * ldci];
-                    if constexpr (CP) { v.x -= acc[0][a][b][h]; v.y -= acc[1][a][b][h]; }
-                    else v -= acc[0][a][b][h];
-                    if (om.col) Cout[(gm < om.nslot ? om.slot + gm : om.tau + (gm - om.nslot)) + om.col[gn] * ldco] = v;
-                    else Cout[gm + gn * ldco] = v;
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int64_t gn = n0 + wn * 16 + b * 8 + 2 * (lane & 3) + h;
+                    v[a][b][h] = gm < M && gn < N ? Cin[gi + gn * ldci] : VT<T>::zero();
                 }
-            }
+        }
+#pragma unroll
+        for (int a = 0; a < AB; a++)
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int64_t gm = m0 + wm * 32 + (a0 + a) * 8 + (lane >> 2);
+                    const int64_t gn = n0 + wn * 16 + b * 8 + 2 * (lane & 3) + h;
+                    if (gm < M && gn < N) {
+                        T x = v[a][b][h];
+                        if constexpr (CP) { x.x -= acc[0][a0 + a][b][h]; x.y -= acc[1][a0 + a][b][h]; }
+                        else x -= acc[0][a0 + a][b][h];
+                        if (om.col) Cout[(gm < om.nslot ? om.slot + gm : om.tau + (gm - om.nslot)) + om.col[gn] * ldco] = x;
+                        else Cout[gm + gn * ldco] = x;
+                    }
+                }
+    }
 }
-
-
 
 // asynchronous global -> shared copies of one element (cp.async: all of a thread's copies in flight at once; completed
 // by cp_async_wait_all, then a barrier).  Both addresses aligned to the element size.
