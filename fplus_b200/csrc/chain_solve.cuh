@@ -13,9 +13,10 @@
 //              cooperative launch.
 //   k_chain_l  L (TR 0) or L^T (TR 1, 2) by one CTA per group of right-hand sides, the front's row vector in shared
 //              memory from front to front (no global round trip), L streamed in 16-column pieces.
-// Both solve a front's triangle by 16 x 16 diagonal blocks inverted once per factorization: four dependent products instead
-// of 64 dependent steps.  All streams are bulk copies (cp.async.bulk) of contiguous, packed pieces: element-wise cp.async
-// issued 26 cycles a warp and held the shared-memory loads of the chain up behind it (a 16 x 16 product took 2,800 cycles).
+// Both solve a front's triangle by 16 x 16 diagonal blocks (diag_solve): one product with the inverted block where that is as
+// accurate as the 16 steps of a substitution, else the substitution.  All streams are bulk copies (cp.async.bulk) of
+// contiguous, packed pieces: element-wise cp.async issued 26 cycles a warp and held the shared-memory loads of the chain up
+// behind it (a 16 x 16 product took 2,800 cycles).
 #pragma once
 #include "kernels.cuh"
 
@@ -24,7 +25,7 @@ namespace fpl {
 constexpr int CH_THREADS = 256, CH_NB = 64, CH_MAXNR = 256, CH_STAGES = 3, CH_UTHREADS = CH_THREADS + 64;
 constexpr unsigned CH_SPIN = 1u << 22;          // polls before a wait for another CTA gives up (about a second)
 constexpr long long CH_CYCLES = 4000000000ll;   // the longest wait for a bulk copy (about two seconds)
-constexpr int CH_BLK = CH_NB * CH_NB + 2;       // a ring stage (two elements more: see chain_ublock)
+constexpr int CH_BLK = CH_NB * CH_NB + 2;       // a ring stage (two elements more: see load_block)
 
 // a chain front as the sweeps read it; nslot, slot, tau: where the previous chain front's contribution rows enter (its row t
 // at initial row slot + t, t < nslot, or tau + t - nslot); u_pk, l_pk: its packed pieces
@@ -32,13 +33,26 @@ struct ChainFront {
     long long f, np, nr, row_off, nslot, slot, tau, u_pk, l_pk;
 };
 
-// Packed pieces of a front's triangles, one per 16 pivots (block b, k0 = 16 b): the inverted diagonal block (256 elements,
-// column-major, identity beyond the front's pivots), then the 16 columns' other entries (zero beyond the pivots):
+// Packed pieces of a front's triangles, one per 16 pivots (block b, k0 = 16 b): the diagonal block (256 elements, element
+// (i, k) at pk_e(i, k): rows and columns both read without bank conflicts), then the 16 columns' other entries (zero beyond
+// the pivots):
 //   U piece b: rows [0, k0) of U11's columns (leading dimension k0), at u_pk + pk_u(b)
 //   L piece b: rows [k0 + w, R) of L's columns (w pivots in the block, leading dimension R - k0 - w), at l_pk + pk_l(b, R);
 //              R = the front's rows on the dense chain, its pivots elsewhere
+// The diagonal block is kept as its inverse D (identity beyond the pivots) or as the triangle itself (U: with the reciprocals
+// of the pivots on its diagonal; one beyond the pivots); which, says the far corner of the other triangle (pk_flag: zero for
+// the inverse).  x = D y leaves a residual of at most about u |U| |D| |U| |x| where substitution leaves u |U| |x|, so the inverse
+// stands only where || |U| |D| ||_1 <= PACK_GROWTH.  Backward errors of x = D y, blocks with a column within 1 to 1e-8.5 of the
+// ones before it: at most 1e-17 times that norm (4e-15 at 1,000, 3e-9 at 3e8; substitution 6e-17 throughout).  The norm (of
+// |re| + |im|) is 2 to 9 on the stencils' and the random matrices' fronts; on the pencils' chains 45 to 50 in the middle (U) and
+// at most 81 (L), about 4 blocks of 100 above 128; on a narrow complex band's 124 in the middle.
 __host__ __device__ constexpr int64_t pk_u(int64_t b) { return 256 * b + 128 * b * (b - 1); }
 __host__ __device__ constexpr int64_t pk_l(int64_t b, int64_t R) { return 256 * b + 16 * b * R - 128 * b * (b + 1); }
+__host__ __device__ constexpr int pk_e(int i, int k) { return 16 * k + ((i + k) & 15); }
+__host__ __device__ constexpr int pk_flag(bool lower) { return lower ? pk_e(0, 15) : pk_e(15, 0); }
+constexpr double PACK_GROWTH = 128.0;
+__device__ __forceinline__ double abs1(double v) { return fabs(v); }
+__device__ __forceinline__ double abs1(cplx v) { return fabs(v.x) + fabs(v.y); }
 
 template <typename T>
 __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ fr, const int *__restrict__ dfront, const T *__restrict__ La,
@@ -51,10 +65,10 @@ __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const T *L = La + F.L_off;
     T *du = pk + F.u_pk + pk_u(b), *dl = pk + F.l_pk + pk_l(b, F.l_rows);
-    if (warp == 0) {                                    // the inverses: a lane per column (U's, then L's)
+    if (warp == 0) {                                    // the diagonal blocks: a lane per column (U's, then L's)
         const int lower = lane >> 4, c = lane & 15;
         T x[16];
-        auto at = [&](int i, int k) -> T { return k0 + i < np && k0 + k < np ? L[(k0 + i) + (int64_t)(k0 + k) * F.nr] : VT<T>::zero(); };
+        auto at = [&](int i, int k) -> T { return i < w && k < w ? L[(k0 + i) + (int64_t)(k0 + k) * F.nr] : VT<T>::zero(); };
         if (lower) {
 #pragma unroll
             for (int i = 0; i < 16; i++) {
@@ -70,12 +84,26 @@ __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ 
 #pragma unroll
                 for (int k = 15; k > i; k--) s = msub(s, at(i, k), x[k]);
                 const T d = at(i, i);                   // (never zero: the factorization reports such a column as singular)
-                x[i] = k0 + i < np ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
+                x[i] = i < w ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
             }
         }
-        T *o = (lower ? dl : du) + c * 16;
+        // the norm: the column sums of the block's moduli times the moduli of the inverse's column, the largest column
+        double cs = lower || c >= w ? 1.0 : 0.0, g = 0.0;
+        for (int i = lower ? c + 1 : 0; i < (lower ? 16 : c + 1); i++) cs += abs1(at(i, c));
 #pragma unroll
-        for (int i = 0; i < 16; i++) o[i] = x[i];
+        for (int i = 0; i < 16; i++) g += __shfl_sync(0xffffffffu, cs, i, 16) * abs1(x[i]);
+        const unsigned good = __ballot_sync(0xffffffffu, g <= PACK_GROWTH);     // (not where the inverse overflows: NaN, infinity)
+        const bool inv = (lower ? good >> 16 : good & 0xffffu) == 0xffffu;
+        T *o = lower ? dl : du;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            if (!inv) {
+                x[i] = (lower ? i > c : i < c) ? at(i, c) : VT<T>::zero();
+                if (!lower && i == c) { const T d = at(c, c); x[i] = c >= w ? VT<T>::one() : is_zero(d) ? VT<T>::zero() : recip(d); }
+                if (lower ? i == 0 && c == 15 : i == 15 && c == 0) x[i] = VT<T>::one();      // (pk_flag)
+            }
+            o[pk_e(i, c)] = x[i];
+        }
     }
     const int rl = (int)F.l_rows - k0 - w;
     for (int c = warp; c < 16; c += 4) {
@@ -184,6 +212,68 @@ __device__ __forceinline__ void quad_mv(T (&acc)[RB], const T *Mp, int ld, int o
     quad_sum<T, RB>(acc);
 }
 
+// x = M^-1 y for a packed 16 x 16 diagonal block D of w <= 16 unknowns: M = L (unit lower) or U (TR 0), or its transpose (TR 1, 2
+// with conj); BACK: M is upper triangular; UNIT: it has a unit diagonal.  y: [k * RB + r], finite or not, zero from w on or not
+// part of the block.  By the threads tid < diag_threads(RB); put(o, r, x) takes unknown o < 16 of right-hand side r, zero from
+// w on (INPLACE: after every thread has read y; named barrier 2).
+//
+// What bounds it (B200, one right-hand side, from y in shared memory to x there, two barriers included): the product 263
+// cycles real, 461 complex; the substitution, a lane per unknown and one exchange per step, 970 (unit) and 1,480 real, 1,630
+// and 1,890 complex (a dependent FP64 operation takes about 25 cycles, a shuffle 27).  Four unknowns at a time, solved by every
+// lane for itself, took 1,180 to 1,200 real and 1,780 to 1,890 complex; the whole block in one lane 960 to 3,080.
+__host__ __device__ constexpr int sub_warps(int rb) { return (rb + 1) / 2; }
+__host__ __device__ constexpr int diag_threads(int rb) { return 32 * sub_warps(rb) > 64 ? 32 * sub_warps(rb) : 64; }
+__device__ __forceinline__ double shfl16_v(double v, int src) { return __shfl_sync(0xffffffffu, v, src, 16); }
+__device__ __forceinline__ cplx shfl16_v(cplx v, int src) { return cplx{shfl16_v(v.x, src), shfl16_v(v.y, src)}; }
+// the substitution (its own function: the product's path keeps the registers): unknown o = tid % 16 of two right-hand sides
+// per warp
+template <typename T, int TR, bool BACK, bool UNIT, int RB>
+__device__ __noinline__ T diag_sub(const T *D, int w, const T *y)
+{
+    auto at = [&](int i, int k) -> T { return TR == 0 ? D[pk_e(i, k)] : opv<TR>(D[pk_e(k, i)]); };
+    const int o = threadIdx.x & 15, r = RB == 1 ? 0 : 2 * (threadIdx.x >> 5) + ((threadIdx.x >> 4) & 1);
+    T a = o < w ? y[o * RB + r] : VT<T>::zero();
+    const T inv = UNIT ? VT<T>::one() : at(o, o);
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+        const int k = BACK ? 15 - s : s;
+        const T x = UNIT ? a : mul(a, inv), v = shfl16_v(x, k), u = msub(a, at(o, k), v);
+        a = o == k ? x : (BACK ? o < k : o > k) ? u : a;
+    }
+    return o < w ? a : VT<T>::zero();
+}
+template <typename T, int TR, bool BACK, bool UNIT, int RB, bool INPLACE, typename PUT>
+__device__ __forceinline__ void diag_solve(const T *D, int w, const T *y, PUT put)
+{
+    const int tid = threadIdx.x;
+    if (is_zero(D[pk_flag((TR == 0) != BACK)])) {
+        if (tid >= 64) return;
+        // four lanes per unknown; the terms outside the triangle are left out, not multiplied by zero (an infinity in y
+        // reaches the unknowns that depend on it, as in a substitution)
+        const int o = quad_o(tid), q = quad_q(tid);
+        T a[RB];
+#pragma unroll
+        for (int r = 0; r < RB; r++) a[r] = VT<T>::zero();
+#pragma unroll
+        for (int z = 0; z < 4; z++) {
+            const int k = 8 * (q & 1) + 4 * (q >> 1) + z;         // (no bank conflicts in either order)
+            const T m = TR == 0 ? D[pk_e(o, k)] : opv<TR>(D[pk_e(k, o)]);
+            const bool in = BACK ? k >= o && k < w : k <= o;
+#pragma unroll
+            for (int r = 0; r < RB; r++) a[r] = madd<T>(a[r], m, in ? y[k * RB + r] : VT<T>::zero());
+        }
+        quad_sum<T, RB>(a);
+        if (INPLACE) named_bar(2, 64);
+        if (q == 0)
+#pragma unroll
+            for (int r = 0; r < RB; r++) put(o, r, o < w ? a[r] : VT<T>::zero());
+        return;
+    }
+    if (tid >= 32 * sub_warps(RB)) return;
+    const T x = diag_sub<T, TR, BACK, UNIT, RB>(D, w, y);
+    if (RB > 1 || tid < 16) put(tid & 15, RB == 1 ? 0 : 2 * (tid >> 5) + ((tid >> 4) & 1), x);
+}
+
 // right-hand sides per pass of the multiple-right-hand-side forms
 template <typename T> __host__ __device__ constexpr int ch_rb() { return VT<T>::cplx_ ? 4 : 8; }
 // dynamic shared memory of k_chain_u for `own` blocks' sums per worker (the larger of the two roles)
@@ -194,12 +284,13 @@ static inline size_t chain_u_smem(int64_t own, int64_t rb, int64_t vs)
     return worker > solver ? worker : solver;
 }
 
-// x = U11^-1 y (TR 0) or U11^-T y of one chain front from its packed pieces tr, by CH_THREADS threads (o, q: quad_o, quad_q;
-// ys and x: [k * RB + r], zero beyond the pivots; ys is overwritten); ends without a barrier after the last writes of x but
+// x = U11^-1 y (TR 0) or U11^-T y of one chain front (np pivots) from its packed pieces tr, by CH_THREADS threads (o, q: quad_o,
+// quad_q; ys and x: [k * RB + r], zero beyond the pivots; ys is overwritten); ends without a barrier after the last writes of x but
 // the named barrier 1 of its steps
 template <typename T, int TR, int RB>
-__device__ __forceinline__ void chain_tri(const T *tr, T *ys, T *x, int nbk, int o, int q)
+__device__ __forceinline__ void chain_tri(const T *tr, T *ys, T *x, int np, int o, int q)
 {
+    const int nbk = (np + 15) >> 4;
     T a[RB];
     for (int bb = 0; bb < nbk; bb++) {
         const int b = TR == 0 ? nbk - 1 - bb : bb, k0 = 16 * b;
@@ -214,12 +305,9 @@ __device__ __forceinline__ void chain_tri(const T *tr, T *ys, T *x, int nbk, int
             }
             named_bar(1, CH_THREADS);
         }
-        if (o < 16) {                              // (beyond the pivots: identity times zero)
-            quad_mv<T, TR, RB>(a, D, 16, o, q, 16, ys + k0 * RB);
-            if (q == 0)
-#pragma unroll
-                for (int r = 0; r < RB; r++) x[(k0 + o) * RB + r] = a[r];
-        }
+        if (threadIdx.x < diag_threads(RB))
+            diag_solve<T, TR, TR == 0, false, RB, false>(D, np - k0 < 16 ? np - k0 : 16, ys + k0 * RB,
+                                                         [&](int i, int r, T v) { x[(k0 + i) * RB + r] = v; });
         named_bar(1, CH_THREADS);
         if (TR == 0 && b > 0) {
             // y[0 .. 16b) -= U[0 .. 16b, b] x_b
@@ -255,8 +343,8 @@ __device__ __forceinline__ void block_mv(T (&a)[RB], const T *M, int nb, int oo,
 // solution; both n x nrhs.  sync[0]: blocks solved; sync[1 + t]: block t has every product but that of block t - 1.
 // rb <= RB right-hand sides.
 //
-// What bounds it: at small K the solver's step (the 64 x 64 product with the block just solved, then four 16 x 16 products
-// and their updates) and the round trip solver - worker - solver; at large K the stream of U12.
+// What bounds it: at small K the solver's step (the 64 x 64 product with the block just solved, then four 16 x 16
+// solves and their updates) and the round trip solver - worker - solver; at large K the stream of U12.
 template <typename T, int TR, int RB>
 __global__ void __launch_bounds__(CH_UTHREADS) k_chain_u(const ChainFront *__restrict__ fr, int K, int nb, int64_t f0, int64_t U0,
                                                          int np_last, const T *__restrict__ Ua, const T *__restrict__ pk, T *Y, T *X,
@@ -426,7 +514,7 @@ __global__ void __launch_bounds__(CH_UTHREADS) k_chain_u(const ChainFront *__res
     };
     if (tid == CH_THREADS - 1) load(0);
     for (int t = 0; t < K; t++) {
-        const int sl = t & 1, np = np_of(t), nbk = (np + 15) >> 4;
+        const int sl = t & 1, np = np_of(t);
         T *ys = yin + sl * CH_NB * RB, *x = xs + sl * CH_NB * RB;
         const T *xp = xs + (sl ^ 1) * CH_NB * RB;
         if (tid == CH_THREADS - 1) load(t + 1);        // (into the stage that block t - 1 used: everyone is past it)
@@ -448,7 +536,7 @@ __global__ void __launch_bounds__(CH_UTHREADS) k_chain_u(const ChainFront *__res
                 for (int r = 0; r < RB; r++) ys[o * RB + r] = sub(ys[o * RB + r], a[r]);
         }
         named_bar(1, CH_THREADS);
-        chain_tri<T, TR, RB>(tri + sl * 2560, ys, x, nbk, o, q);
+        chain_tri<T, TR, RB>(tri + sl * 2560, ys, x, np, o, q);
         named_arrive(4 + (t & 1), CH_THREADS + 32);    // x is in shared memory: out it goes (two barriers in turn: block t + 2
                                                        // cannot be done before block t is out)
     }
@@ -522,7 +610,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_chain_ustep(const ChainFront *__
     }
     if (blockIdx.x > 0) return;
     __syncthreads();
-    chain_tri<T, TR, RB>(tr, ys, x, (np + 15) >> 4, o, q);
+    chain_tri<T, TR, RB>(tr, ys, x, np, o, q);
     __syncthreads();
     for (int e = tid; e < np * rb; e += CH_THREADS) { const int k = e % np, r = e / np; X[f_of(t) + k + r * n] = x[k * RB + r]; }
 }
@@ -617,17 +705,12 @@ __global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__rest
                 return;
             }
             const T *D = ring + (done % CH_LSTAGES) * psz, *Lp = D + 256;      // Lp[c * rl + (row - k0 - w)]
-            T a[RB];
             if (TR == 0) {
-                if (tid < 64) {
-                    quad_mv<T, 0, RB>(a, D, 16, quad_o(tid), quad_q(tid), 16, v + k0 * RB);   // (past the pivots: zero columns of the inverse's rows)
-                    named_bar(2, 64);
-                    if (quad_q(tid) == 0 && quad_o(tid) < w) {
-                        const int oo = quad_o(tid);
-#pragma unroll
-                        for (int r = 0; r < RB; r++) { v[(k0 + oo) * RB + r] = a[r]; if (r < rb) S2[F.f + k0 + oo + r * n] = a[r]; }
-                    }
-                } else if (loader) load_next();
+                if (tid < diag_threads(RB))
+                    diag_solve<T, 0, false, true, RB, true>(D, w, v + k0 * RB, [&](int i, int r, T a) {
+                        if (i < w) { v[(k0 + i) * RB + r] = a; if (r < rb) S2[F.f + k0 + i + r * n] = a; }
+                    });
+                else if (loader) load_next();
                 // the next front's rows, a block step after the load each needs (so that none waits)
                 if (bb == (nbk > 1 ? 1 : 0) && pm >= 0) {
                     t = pm >= gsl && pm < gsl + gns ? pm - gsl : pm >= gta ? gns + pm - gta : -1;
@@ -676,25 +759,10 @@ __global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__rest
                     if (c < w && l16 == 0) v[(k0 + c) * RB + r] = sub(v[(k0 + c) * RB + r], s[r]);
                 }
                 __syncthreads();
-                if (tid < 64) {
-                    // (a last block of fewer than 16 pivots: the rows after it are not part of it)
-                    const int oo = quad_o(tid), q = quad_q(tid);
-#pragma unroll
-                    for (int r = 0; r < RB; r++) a[r] = VT<T>::zero();
-#pragma unroll
-                    for (int z = 0; z < 4; z++) {
-                        const int kq = (4 * q + z + oo) & 15;
-                        const T m = opv<TR>(D[oo * 16 + kq]);
-                        if (kq < w)
-#pragma unroll
-                            for (int r = 0; r < RB; r++) a[r] = madd<T>(a[r], m, v[(k0 + kq) * RB + r]);
-                    }
-                    quad_sum<T, RB>(a);
-                    named_bar(2, 64);
-                    if (q == 0 && oo < w)
-#pragma unroll
-                        for (int r = 0; r < RB; r++) { v[(k0 + oo) * RB + r] = a[r]; if (r < rb) S2[F.f + k0 + oo + r * n] = a[r]; }
-                }
+                if (tid < diag_threads(RB))
+                    diag_solve<T, TR, true, true, RB, true>(D, w, v + k0 * RB, [&](int i, int r, T a) {
+                        if (i < w) { v[(k0 + i) * RB + r] = a; if (r < rb) S2[F.f + k0 + i + r * n] = a; }
+                    });
             }
         }
         if (!more) break;

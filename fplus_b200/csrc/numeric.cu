@@ -1325,7 +1325,7 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
     const T *La = (const T *)N.Larena, *Ua = (const T *)N.Uarena;
     const int64_t nf = (int64_t)P.fronts.size();
     const int64_t nlev = (int64_t)D.sv_rows_ptr.size() - 1;
-    // The dense chain's sweeps in one launch each where its fronts qualify (upload_plan) and the block inverses are there;
+    // The dense chain's sweeps in one launch each where its fronts qualify (upload_plan);
     // measured against a launch per front: see the kernels' comments
     const bool one_chain = D.ch_count > 0;
     const T *PK = (const T *)N.pk;

@@ -95,7 +95,7 @@ struct DevNum {
     size_t cap_perm = 0;
     int *permall = nullptr;        // every front's final row order (position -> initial local row), kept for the solves
     size_t cap_permall = 0;
-    void *pk = nullptr;            // the fronts' packed triangles with inverted 16 x 16 diagonal blocks (k_front_pack)
+    void *pk = nullptr;            // the fronts' packed triangles by 16-column pieces (k_front_pack)
     unsigned *chsync = nullptr;    // the dense chain's sweeps' counters, its workers' sums
     void *chacc = nullptr;
     size_t cap_pk = 0, cap_chsync = 0, cap_chacc = 0;

@@ -8,7 +8,7 @@ constexpr int SW_THREADS = 256;
 
 // A front's triangle applied to the vector x (x[k * RB + r], k up to np and zero from there to the next sixteen, shared
 // memory; overwritten), the result in xs (the same layout): xs = L11^-1 x (UPPER false) or U11^-1 x.  By 16-column blocks: the
-// block's 16 unknowns as one product with the inverted diagonal block, then the rows beyond it updated from the block's
+// block's 16 unknowns (diag_solve), then the rows beyond it updated from the block's
 // columns; the packed pieces (at pk, see k_front_pack) stream through a ring of STG stages of psz elements by bulk copies
 // ahead of the chain.  The pipe (its barriers, initialised, and the pieces taken so far) serves several calls of a CTA of
 // SW_THREADS.  Ends with a barrier; false (for every thread) when a copy did not land.
@@ -38,13 +38,8 @@ __device__ __forceinline__ bool tri16(const T *__restrict__ pk, int np, T *x, T 
         __syncthreads();                               // (the piece before is no longer read; x is as its updates left it)
         const T *D = ring + (d % STG) * psz, *Lp = D + 256;
         if (tid == SW_THREADS - 1) load_next();
-        if (tid < 64) {
-            T a[RB];
-            quad_mv<T, 0, RB>(a, D, 16, quad_o(tid), quad_q(tid), 16, x + k0 * RB);
-            if (quad_q(tid) == 0)
-#pragma unroll
-                for (int r = 0; r < RB; r++) xs[(k0 + quad_o(tid)) * RB + r] = a[r];
-        }
+        if (tid < diag_threads(RB))
+            diag_solve<T, 0, UPPER, !UPPER, RB, false>(D, w, x + k0 * RB, [&](int i, int r, T v) { xs[(k0 + i) * RB + r] = v; });
         __syncthreads();
         // the rows beyond the block: two lanes per row, eight columns each (columns beyond the pivots are zero)
         const int ra = UPPER ? 0 : k0 + w, rl = UPPER ? k0 : np - k0 - w;

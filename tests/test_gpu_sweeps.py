@@ -1,10 +1,11 @@
-"""The sweeps by inverted 16 x 16 diagonal blocks at the sizes where they can go wrong: the dense chain in one launch (a last
+"""The sweeps by packed 16-column pieces at the sizes where they can go wrong: the dense chain in one launch (a last
 block of one pivot, partial 16-blocks, 32- and 64-pivot fronts, one and several blocks per worker, the cluster and the
 cooperative form) and the level-scheduled sweeps of the other fronts (narrow and wide fronts, the widest on the 64-row
 substitution), for one right-hand side, the edges of a pass of eight, and every trans.  The bar is the parity tests': backward
 error at most 1e-14."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import fplus_b200 as F
 from fplus_b200 import workloads as W
@@ -83,3 +84,78 @@ def test_levels(gpu, cplx, width):
     for trans in (0, 1):
         for nrhs in (1, 3, 8, 9, 33 if width < 512 else 17):     # (the widest fronts' vectors must fit one CTA: fewer at once)
             _check(m, S, N, nrhs, trans)
+
+
+def _hard(kind, n, cplx, seed):
+    """A dense matrix whose triangles hold 16 x 16 diagonal blocks with large inverses; what else it needs."""
+    rng = np.random.default_rng(seed)
+    i, j = np.indices((n, n))
+    if kind.startswith("dependent"):           # columns within delta of a combination of the ones before them
+        delta = float(kind.split(":")[1])
+        A = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0)
+        for c in (5, 15, 20, 37):
+            A[:, c] = A[:, :c] @ rng.uniform(-1, 1, c) + delta * A[:, c]
+    elif kind == "vandermonde":
+        A = np.linspace(0.0, 1.0, n)[:, None] ** np.arange(n)
+    elif kind == "kernel":
+        t = np.linspace(0.0, 1.0, n)
+        A = np.exp(-4.0 * (t[:, None] - t) ** 2)
+    elif kind == "upper":                       # U = A
+        A = np.where(i == j, 0.1, np.where((j > i) & (j // 16 == i // 16), -1.0, 0.0))
+    else:                                       # "lower": L = A, multipliers of one
+        A = np.where(i == j, 1.0, np.where((j < i) & (j // 16 == i // 16), -1.0, 0.0))
+    if cplx:
+        A = A * np.exp(0.7j)
+    return n, np.arange(n + 1, dtype=np.int64) * n, np.tile(np.arange(n, dtype=np.int64), n), np.ascontiguousarray(A.T).ravel()
+
+
+def _check_from_x(m, N, nrhs, trans):
+    """b = op(A) x with a moderate x (a random b lets x grow along the small directions, which hides a large residual)."""
+    n, Ap, Ai, Ax = m
+    rng = np.random.default_rng(11 + nrhs)
+    A = sp.csc_matrix((Ax, Ai, Ap), shape=(n, n))
+    x = rng.uniform(-1, 1, (n, nrhs)) + (1j * rng.uniform(-1, 1, (n, nrhs)) if np.iscomplexobj(Ax) else 0)
+    b = np.asarray({0: A, 1: A.T, 2: A.conj().T}[trans] @ x)
+    y = N.solve(b, trans)
+    worst = max(O.backward_error(n, Ap, Ai, Ax, y[:, r], b[:, r], trans) for r in range(nrhs))
+    assert worst <= 1e-14, (nrhs, trans, worst)
+
+
+@pytest.mark.parametrize("kind,n", [("dependent:1e-4", 64), ("dependent:1e-7", 64), ("dependent:1e-7", 180), ("vandermonde", 16),
+                                    ("kernel", 32), ("upper", 16), ("upper", 180), ("lower", 48), ("lower", 180)])
+@pytest.mark.parametrize("where", ["tree", "chain"])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_ill_conditioned_diagonal_blocks(gpu, cplx, where, kind, n):
+    """The backward error of a solve does not depend on the conditioning of the triangles' diagonal blocks: fronts of the
+    tree (np <= 64 and wider), and the dense chain (every row taken as dense)."""
+    m = _hard(kind, n, cplx, 4)
+    eye = np.arange(n, dtype=np.int64)
+    S = F.Symbolic.from_orders(*m[:3], eye, eye) if where == "chain" else F.analyze(*m[:3], pin_dense=0)
+    assert np.array_equal(S.col_perm, eye) and np.array_equal(S.row_perm, eye)
+    N = S.factor(m[3], F.default_options(equilibrate=0, pivot_rel=0.0, pin_dense=0))
+    assert N.info["f_dense"] == (0 if where == "chain" else n)
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        for nrhs in (1, 3, 9):
+            _check_from_x(m, N, nrhs, trans)
+
+
+@pytest.mark.parametrize("delta", [1e-4, 1e-7])
+@pytest.mark.parametrize("nb", [32, 64])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_ill_conditioned_chain(gpu, cplx, nb, delta):
+    """The same on the dense chain: columns all along it that depend on the two before them to delta."""
+    n, Ap, Ai, Ax = _band(500, cplx, 8, hbw=5, ntau=3)
+    A = sp.csc_matrix((Ax, Ai, Ap), shape=(n, n)).tolil()
+    for c in range(40, n - 3, 23):
+        A[:, c] = 0.7 * A[:, c - 1] - 0.4 * A[:, c - 2] + delta * A[:, c]
+    A = A.tocsc()
+    A.sort_indices()
+    m = n, A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data.copy()
+    eye = np.arange(n, dtype=np.int64)
+    S = F.Symbolic.from_orders(*m[:3], eye, eye)
+    S.set_front_shape(256, nb, 2)
+    N = S.factor(m[3])
+    assert N.info["f_dense"] < 200
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        for nrhs in (1, 9):
+            _check_from_x(m, N, nrhs, trans)
