@@ -668,10 +668,14 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
                  mc_ub = r256((size_t)(P.max_npiv > 0 ? P.max_npiv : 1) * (P.max_npiv > 0 ? P.max_npiv : 1) * vs),
                  mc_mark = r256((size_t)(P.max_nrows > 0 ? P.max_nrows : 1) * 4), mc_rid = r256((size_t)(P.max_nrows > 0 ? P.max_nrows : 1) * 8);
     bool any_mc = false;
-    // the cluster form also takes the blocks that one CTA holds but the panel LU does not (300 and more rows of 64 columns):
-    // a step costs 0.6 us there against 2 us and more in k_front_lu2
+    // the cluster form also takes most of the blocks that one CTA holds but the panel LU does not.  Measured, the final order
+    // included (us, cluster / k_front_lu2): real 332 x 64 80.9 / 137.2, 700 x 32 46.1 / 93.4, 200 x 128 151 / 336, 150 x 150
+    // 179 / 426; complex 196 x 64 118.6 / 157.9, 252 x 48 91.8 / 111.0, 140 x 96 171.7 / 266.5, 228 x 32 62.9 / 66.2, 260 x 16
+    // 35.5 / 37.8.  But complex blocks of at most 128 rows, and of at most 16 columns below 256 rows, stay: 108 x 108 193 / 170,
+    // 116 x 116 213 / 200, 244 x 16 35.1 / 34.1
     auto takes_mc = [&](int64_t nr, int64_t np) {
-        return front_lu_smem(nr, np, vs) > SMEM_MAX || ((N.lu_variant & 7) == 2 && mc_cl > 0 && !front_lu6_fits<T>(nr, np) && nr >= np && np > 0 && nr >= 64);
+        return front_lu_smem(nr, np, vs) > SMEM_MAX || ((N.lu_variant & 7) == 2 && mc_cl > 0 && !front_lu6_fits<T>(nr, np) && nr >= np && np > 0 &&
+                                                        nr >= (!N.cplx ? 64 : np > 16 ? 129 : 256));
     };
     for (const Front &F : P.fronts)
         if (takes_mc(F.nrows, F.npiv)) { any_mc = true; break; }

@@ -55,7 +55,7 @@ def _check(m, equilibrate=1, variant=2):
     assert _rel(L, orc.L) <= FACTOR_TOL and _rel(U, orc.U) <= FACTOR_TOL
 
 
-@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33, 63, 65, 96, 127, 128, 129, 145])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33, 63, 65, 96, 109, 116, 127, 128, 129, 145])
 @pytest.mark.parametrize("cplx", [False, True])
 def test_sizes(gpu, cplx, n):
     _check(_dense(n, cplx, n))
