@@ -1229,6 +1229,25 @@ static int chain_row_sweep(const FrontPlan &P, const DevPlan &D, DevNum &N, cons
         (int)nrhs, N.st), note_launch();
     return FPLUS_OK;
 }
+// the column sweep by a launch per step, for captured graphs
+template <typename T, int TR, int RB>
+static int chain_col_steps(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, char *err, size_t errlen)
+{
+    const int K = (int)D.ch_count;
+    const size_t sm = chain_ustep_smem(RB, sizeof(T));
+    int rc;
+    if ((rc = ensure_async(N, &N.chacc, &N.cap_chacc, (size_t)(D.ch_count * CH_NB * RB) * sizeof(T), err, errlen))) return rc;
+    CK(cudaFuncSetAttribute(k_chain_ustep<T, TR, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    for (int64_t r0 = 0; r0 < nrhs; r0 += RB)
+        for (int s = -1; s < K - 1; s++) {
+            CK(launch_pdl(k_chain_ustep<T, TR, RB>, 1 + std::max(0, s >= 0 ? K - 2 - s : 0), CH_THREADS, sm, N.stream, (const ChainFront *)D.ch_fronts,
+                          K, (int)D.chain_nb, D.chain_f0, D.ch_u0, (int)D.ch_nplast, (const T *)N.Uarena, (const T *)N.pk, Y + r0 * N.n,
+                          X + r0 * N.n, N.n, (int)std::min<int64_t>(RB, nrhs - r0), s, (T *)N.chacc, (const DevStatus *)N.st));
+            note_launch();
+        }
+    return FPLUS_OK;
+}
+// the column sweep in one cooperative launch per pass
 template <typename T, int TR, int RB>
 static int chain_col_sweep(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, int64_t G, char *err, size_t errlen)
 {
@@ -1249,27 +1268,14 @@ static int chain_col_sweep(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs
         DevStatus *st = N.st;
         T *ga = wide ? (T *)N.chacc : nullptr;
         void *args[] = {&fr, &Ki, &nb, &f0, &U0, &npl, &Ua, &pk, &Yr, &Xr, &n, &m, &sy, &ga, &st};
-        CK(cudaLaunchCooperativeKernel((const void *)k_chain_u<T, TR, RB>, (unsigned)G, CH_UTHREADS, args, sm, N.stream));
+        const cudaError_t le = cudaLaunchCooperativeKernel((const void *)k_chain_u<T, TR, RB>, (unsigned)G, CH_UTHREADS, args, sm, N.stream);
+        if (le == cudaErrorCooperativeLaunchTooLarge) {      // (fewer SMs at hand than the device has: nothing has run)
+            (void)cudaGetLastError();
+            return chain_col_steps<T, TR, RB>(D, N, Yr, Xr, nrhs - r0, err, errlen);
+        }
+        CK(le);
         note_launch();
     }
-    return FPLUS_OK;
-}
-// the same by a launch per step, for captured graphs
-template <typename T, int TR, int RB>
-static int chain_col_steps(const DevPlan &D, DevNum &N, T *Y, T *X, int64_t nrhs, char *err, size_t errlen)
-{
-    const int K = (int)D.ch_count;
-    const size_t sm = chain_ustep_smem(RB, sizeof(T));
-    int rc;
-    if ((rc = ensure_async(N, &N.chacc, &N.cap_chacc, (size_t)(D.ch_count * CH_NB * RB) * sizeof(T), err, errlen))) return rc;
-    CK(cudaFuncSetAttribute(k_chain_ustep<T, TR, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-    for (int64_t r0 = 0; r0 < nrhs; r0 += RB)
-        for (int s = -1; s < K - 1; s++) {
-            CK(launch_pdl(k_chain_ustep<T, TR, RB>, 1 + std::max(0, s >= 0 ? K - 2 - s : 0), CH_THREADS, sm, N.stream, (const ChainFront *)D.ch_fronts,
-                          K, (int)D.chain_nb, D.chain_f0, D.ch_u0, (int)D.ch_nplast, (const T *)N.Uarena, (const T *)N.pk, Y + r0 * N.n,
-                          X + r0 * N.n, N.n, (int)std::min<int64_t>(RB, nrhs - r0), s, (T *)N.chacc, (const DevStatus *)N.st));
-            note_launch();
-        }
     return FPLUS_OK;
 }
 // U x = y (TR 0: Y in pivot order, x into X) or U^T z = w (in place).  Workers: one per block as far as the SMs go (one SM
