@@ -1,8 +1,8 @@
-"""The sweeps by packed 16-column pieces at the sizes where they can go wrong: the dense chain in one launch (a last
-block of one pivot, partial 16-blocks, 32- and 64-pivot fronts, one and several blocks per worker, the cluster and the
-cooperative form) and the level-scheduled sweeps of the other fronts (narrow and wide fronts, the widest on the 64-row
-substitution), for one right-hand side, the edges of a pass of eight, and every trans.  The bar is the parity tests': backward
-error at most 1e-14."""
+"""The sweeps by packed 16-column pieces at the sizes where they can go wrong: the dense chain in one launch per sweep (a last
+block of one pivot, partial 16-blocks, 8-, 32- and 64-pivot fronts, one and several blocks per worker) and by a launch per
+front (more rows than one CTA takes), and the level-scheduled sweeps of the other fronts (narrow and wide fronts, the widest
+on the 64-row substitution), for one right-hand side, the edges of a pass of eight, and every trans; diagonal blocks that are
+too ill-conditioned for their inverses.  The bar is the parity tests': backward error at most 1e-14."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -63,13 +63,50 @@ def test_chain(gpu, cplx, n, nb):
 
 @pytest.mark.parametrize("n,nb", [(2100, 32), (9300, 64)])
 def test_chain_of_many_blocks(gpu, n, nb):
-    """More than four blocks per worker in one cluster; a cooperative launch."""
+    """Chains of 66 and 146 blocks, a worker CTA per block."""
     m = _band(n, False, n)
     S = F.analyze(*m[:3])
     S.set_front_shape(256, nb, 2)
     N = S.factor(m[3])
     for trans in (0, 1):
         for nrhs in (1, 11):
+            _check(m, S, N, nrhs, trans)
+
+
+@pytest.mark.parametrize("cplx,nrhs", [(False, 1), (False, 9), (True, 1), (True, 5)])
+def test_chain_of_several_blocks_per_worker(gpu, cplx, nrhs):
+    """A chain of about 1,100 blocks of 8 pivots: seven or eight blocks per worker, their sums in shared memory (one
+    right-hand side; real values) or in global memory (complex, several right-hand sides).  The solution equals, bit for bit,
+    that of the launch per step that a captured graph takes, which has a CTA per block."""
+    m = _band(9000, cplx, 6)
+    n = m[0]
+    S = F.analyze(*m[:3])
+    S.set_front_shape(256, 8, 2)
+    N = S.factor(m[3])
+    assert (n - N.info["f_dense"]) // 8 > 7 * 147
+    b = np.asfortranarray(np.random.default_rng(2).standard_normal((n, nrhs)) + (0j if cplx else 0))
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        x = N.solve(b, trans)
+        G = F.BatchGraph([N], nrhs, trans)
+        G.upload(0, m[3], b)
+        G.launch()
+        assert G.status() == [0]
+        assert np.array_equal(G.download(0).reshape(n, nrhs), x.reshape(n, nrhs)), trans
+        for r in range(nrhs):
+            assert O.backward_error(*m, x[:, r], b[:, r], trans) <= 1e-14
+
+
+@pytest.mark.parametrize("ntau", [140, 230])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_wide_chain(gpu, cplx, ntau):
+    """Chain fronts of more than 197 rows, and of more than 256: a launch per front."""
+    m = _band(900, cplx, 5, ntau=ntau)
+    S = F.analyze(*m[:3])
+    N = S.factor(m[3])
+    P = S.plan(N.info["f_dense"])
+    assert N.info["f_dense"] < m[0] and P["nrows"][P["col_front"][N.info["f_dense"]]:].max() > (256 if ntau == 230 else 197)
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        for nrhs in (1, 2, 9):
             _check(m, S, N, nrhs, trans)
 
 
