@@ -2,7 +2,7 @@
 // [f, n), each front's contribution block the next one's only child), and the packed triangles that all sweeps read.
 //
 // The chain is one dependency: K blocks of nb unknowns, each needing every one before it.  The column sweeps (U, U^T) read
-// n^2 / 2 entries of U12 (8.6 GB for n = 32,768 complex), the row sweeps (L, L^T) K blocks of at most 256 x 64.
+// n^2 / 2 entries of U12 (8.6 GB for n = 32,768 complex), the row sweeps (L, L^T) K blocks of at most 197 x 64.
 //
 //   k_chain_u  U x = y (TR 0, from the last front) or U^T z = w (TR 1, 2, from the first): one launch.  CTA 0 solves block
 //              after block; the other CTAs own blocks of unknowns and subtract the solved blocks' products from them as

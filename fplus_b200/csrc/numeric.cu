@@ -113,11 +113,12 @@ static int upload_segments(int64_t n, const std::vector<int64_t> &Bp, DevPlan &D
 // (U, U^T) likewise with its columns and U12; the dense chain's fronts, which the U sweep takes by its own kernels, go
 // with the larger fronts in the column sweeps.
 static const int64_t SV_MAXDIM = 768, SV_MAXNP = 64, SV_MAXBLK = 32768;
-// front fi's packed pieces (k_front_pack): their offsets from *size on, which moves past them, and the rows of its L pieces
+// front fi's packed pieces (k_front_pack): their offsets from *size on, which moves past them, and the rows of its L pieces (all
+// of the front's where the one-launch chain sweeps read them)
 static void pack_layout(const FrontPlan &P, const DevPlan &D, int64_t fi, long long *u_pk, long long *l_pk, long long *l_rows, int64_t *size)
 {
     const Front &F = P.fronts[(size_t)fi];
-    const int64_t np = std::min(F.npiv, F.nrows), nb = (np + 15) / 16, R = D.chain_begin >= 0 && fi >= D.chain_begin ? F.nrows : np;
+    const int64_t np = std::min(F.npiv, F.nrows), nb = (np + 15) / 16, R = D.ch_count > 0 && fi >= D.chain_begin ? F.nrows : np;
     *u_pk = *size;
     *l_pk = *size + pk_u(nb);
     *l_rows = R;
@@ -347,18 +348,15 @@ int dev_upload_plan(const fplus_symbolic *S, const FrontPlan &P, DevPlan &D, cha
             D.chain_begin = c0; D.chain_nb = nb; D.chain_f0 = P.fronts[c0].f;
             if ((rc = upload(uoff, &D.chain_uoff, err, errlen))) return rc;
             // the chain as the one-launch sweeps take it (chain_solve.cuh): every front but the first with the one before
-            // as its only child, the row vector of a front in one CTA
+            // as its only child, the row vector of a front in one CTA (at most CH_MAXNR rows, a thread each, and four of a
+            // complex front's L pieces in shared memory: at most 197 rows)
             std::vector<ChainFront> cf;
             bool one = true, uo_ok = nb % 2 == 0;
             int64_t u_next = P.fronts[c0].U_off;
-            int64_t mnr = 0, pks = 0;
-            long long up = 0, lp = 0, lr = 0;
-            D.chain_begin = c0;
-            for (int64_t j = 0; j < c0; j++) pack_layout(P, D, j, &up, &lp, &lr, &pks);
+            int64_t mnr = 0;
             for (int64_t j = c0; one && j < nf; j++) {
                 const Front &F = P.fronts[j];
-                pack_layout(P, D, j, &up, &lp, &lr, &pks);
-                ChainFront c = {F.f, F.npiv, F.nrows, F.row_off, 0, 0, 0, up, lp};
+                ChainFront c = {F.f, F.npiv, F.nrows, F.row_off, 0, 0, 0, 0, 0};
                 // (U12 blocks one after another, as the column sweep finds them)
                 uo_ok = uo_ok && F.U_off == u_next;
                 u_next += F.npiv * (F.ncols - F.npiv);
@@ -373,6 +371,12 @@ int dev_upload_plan(const fplus_symbolic *S, const FrontPlan &P, DevPlan &D, cha
             }
             if (one && uo_ok && chain_l_smem(mnr, 1, 16) <= 220 * 1024) {
                 D.ch_count = nf - c0; D.ch_maxnr = mnr; D.ch_u0 = P.fronts[c0].U_off; D.ch_nplast = P.fronts[nf - 1].npiv;
+                int64_t pks = 0;
+                long long up = 0, lp = 0, lr = 0;
+                for (int64_t j = 0; j < nf; j++) {
+                    pack_layout(P, D, j, &up, &lp, &lr, &pks);
+                    if (j >= c0) { cf[(size_t)(j - c0)].u_pk = up; cf[(size_t)(j - c0)].l_pk = lp; }
+                }
                 if ((rc = upload(cf, &D.ch_fronts, err, errlen))) return rc;
             }
         }
