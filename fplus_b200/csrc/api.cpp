@@ -200,7 +200,7 @@ static int factor_common(const fplus_symbolic *sym, const int64_t *Ap, const int
         }
         I.nnz_L = nl; I.nnz_U = nu;
         I.front_flops = 2.0 * P->flops_real * (is_complex ? 4.0 : 1.0);
-        I.device_bytes = (int64_t)(N.cap_L + N.cap_U + N.cap_cb + N.cap_work + N.cap_work2 + N.cap_tcws + 2 * bytes);
+        I.device_bytes = (int64_t)(N.cap_L + N.cap_U + N.cap_cb + N.cap_work + N.cap_work2 + N.cap_tcws + N.cap_pk + N.cap_rz + 2 * bytes);
         I.precision = prec;
         I.tc_updates = N.tc_updates;
         I.tc_flops = N.tc_flops;

@@ -196,3 +196,18 @@ def test_ill_conditioned_chain(gpu, cplx, nb, delta):
     for trans in ((0, 1, 2) if cplx else (0, 1)):
         for nrhs in (1, 9):
             _check_from_x(m, N, nrhs, trans)
+
+
+def test_device_bytes_count_the_packed_triangles(gpu):
+    """info's device_bytes hold the factors and the triangles packed for the sweeps (16 x 16 blocks and panels)."""
+    n = 100000
+    k = np.arange(n)
+    A = sp.csc_matrix((np.concatenate([np.full(n, 4.0), np.ones(2 * n - 2)]),
+                       (np.concatenate([k, k[1:], k[:-1]]), np.concatenate([k, k[:-1], k[1:]]))), shape=(n, n))
+    S = F.analyze(n, A.indptr.astype(np.int64), A.indices.astype(np.int64))
+    N = S.factor(A.data)
+    P = S.plan()
+    npiv, nc = np.bincount(P["col_front"]), np.diff(P["col_ptr"])
+    entries = int((P["nrows"] * npiv + npiv * (nc - npiv)).sum())
+    packed = 512 * int((npiv >= 16).sum())          # fronts of one block: its upper and its lower triangle
+    assert N.info["device_bytes"] >= 8 * (entries + packed) + 2 * 8 * A.nnz
