@@ -41,15 +41,17 @@ struct ChainFront {
 //              R = the front's rows on the dense chain, its pivots elsewhere
 // The diagonal block is kept as its inverse D (identity beyond the pivots) or as the triangle itself (U: with the reciprocals
 // of the pivots on its diagonal; one beyond the pivots); which, says the far corner of the other triangle (pk_flag: zero for
-// the inverse).  x = D y leaves a residual of at most about u |U| |D| |U| |x| where substitution leaves u |U| |x|, so the inverse
+// the inverse).  A tree front of at most 8 pivots has a block of 2, 4 or 8 rows and columns (side s) instead of 16: with 256
+// elements for every one-pivot front a diagonal matrix's packed triangles were 512 times its factors.  x = D y leaves a residual of at most about u |U| |D| |U| |x| where substitution leaves u |U| |x|, so the inverse
 // stands only where || |U| |D| ||_1 <= PACK_GROWTH.  Backward errors of x = D y, blocks with a column within 1 to 1e-8.5 of the
 // ones before it: at most 1e-17 times that norm (4e-15 at 1,000, 3e-9 at 3e8; substitution 6e-17 throughout).  The norm (of
 // |re| + |im|) is 2 to 9 on the stencils' and the random matrices' fronts; on the pencils' chains 45 to 50 in the middle (U) and
 // at most 81 (L), about 4 blocks of 100 above 128; on a narrow complex band's 124 in the middle.
 __host__ __device__ constexpr int64_t pk_u(int64_t b) { return 256 * b + 128 * b * (b - 1); }
 __host__ __device__ constexpr int64_t pk_l(int64_t b, int64_t R) { return 256 * b + 16 * b * R - 128 * b * (b + 1); }
-__host__ __device__ constexpr int pk_e(int i, int k) { return 16 * k + ((i + k) & 15); }
-__host__ __device__ constexpr int pk_flag(bool lower) { return lower ? pk_e(0, 15) : pk_e(15, 0); }
+__host__ __device__ constexpr int pk_e(int i, int k, int s = 16) { return s * k + ((i + k) & (s - 1)); }
+__host__ __device__ constexpr int pk_flag(bool lower, int s = 16) { return lower ? pk_e(0, s - 1, s) : pk_e(s - 1, 0, s); }
+__host__ __device__ constexpr int pk_side(int64_t np) { return np > 8 ? 16 : np > 4 ? 8 : np > 2 ? 4 : 2; }
 constexpr double PACK_GROWTH = 128.0;
 __device__ __forceinline__ double abs1(double v) { return fabs(v); }
 __device__ __forceinline__ double abs1(cplx v) { return fabs(v.x) + fabs(v.y); }
@@ -62,7 +64,7 @@ __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ 
     const int64_t blk = blockIdx.x;
     const SvFront F = fr[dfront[blk]];
     const int np = (int)(F.np < F.nr ? F.np : F.nr), b = (int)(blk - F.d_off), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sd = (int)F.pk_s;
     const T *L = La + F.L_off;
     T *du = pk + F.u_pk + pk_u(b), *dl = pk + F.l_pk + pk_l(b, F.l_rows);
     if (warp == 0) {                                    // the diagonal blocks: a lane per column (U's, then L's)
@@ -100,9 +102,9 @@ __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ 
             if (!inv) {
                 x[i] = (lower ? i > c : i < c) ? at(i, c) : VT<T>::zero();
                 if (!lower && i == c) { const T d = at(c, c); x[i] = c >= w ? VT<T>::one() : is_zero(d) ? VT<T>::zero() : recip(d); }
-                if (lower ? i == 0 && c == 15 : i == 15 && c == 0) x[i] = VT<T>::one();      // (pk_flag)
+                if (lower ? i == 0 && c == sd - 1 : i == sd - 1 && c == 0) x[i] = VT<T>::one();      // (pk_flag)
             }
-            o[pk_e(i, c)] = x[i];
+            if (i < sd && c < sd) o[pk_e(i, c, sd)] = x[i];
         }
     }
     const int rl = (int)F.l_rows - k0 - w;
@@ -213,7 +215,7 @@ __device__ __forceinline__ void quad_mv(T (&acc)[RB], const T *Mp, int ld, int o
 }
 
 // x = M^-1 y for a packed 16 x 16 diagonal block D of w <= 16 unknowns: M = L (unit lower) or U (TR 0), or its transpose (TR 1, 2
-// with conj); BACK: M is upper triangular; UNIT: it has a unit diagonal.  y: [k * RB + r], finite or not, zero from w on or not
+// with conj); BACK: M is upper triangular; UNIT: it has a unit diagonal; sd: the block's side (w <= sd).  y: [k * RB + r], finite or not, zero from w on or not
 // part of the block.  By the threads tid < diag_threads(RB); put(o, r, x) takes unknown o < 16 of right-hand side r, zero from
 // w on (INPLACE: after every thread has read y; named barrier 2).
 //
@@ -228,9 +230,9 @@ __device__ __forceinline__ cplx shfl16_v(cplx v, int src) { return cplx{shfl16_v
 // the substitution (its own function: the product's path keeps the registers): unknown o = tid % 16 of two right-hand sides
 // per warp
 template <typename T, int TR, bool BACK, bool UNIT, int RB>
-__device__ __noinline__ T diag_sub(const T *D, int w, const T *y)
+__device__ __noinline__ T diag_sub(const T *D, int sd, int w, const T *y)
 {
-    auto at = [&](int i, int k) -> T { return TR == 0 ? D[pk_e(i, k)] : opv<TR>(D[pk_e(k, i)]); };
+    auto at = [&](int i, int k) -> T { return i < sd && k < sd ? (TR == 0 ? D[pk_e(i, k, sd)] : opv<TR>(D[pk_e(k, i, sd)])) : VT<T>::zero(); };
     const int o = threadIdx.x & 15, r = RB == 1 ? 0 : 2 * (threadIdx.x >> 5) + ((threadIdx.x >> 4) & 1);
     T a = o < w ? y[o * RB + r] : VT<T>::zero();
     const T inv = UNIT ? VT<T>::one() : at(o, o);
@@ -243,10 +245,10 @@ __device__ __noinline__ T diag_sub(const T *D, int w, const T *y)
     return o < w ? a : VT<T>::zero();
 }
 template <typename T, int TR, bool BACK, bool UNIT, int RB, bool INPLACE, typename PUT>
-__device__ __forceinline__ void diag_solve(const T *D, int w, const T *y, PUT put)
+__device__ __forceinline__ void diag_solve(const T *D, int sd, int w, const T *y, PUT put)
 {
     const int tid = threadIdx.x;
-    if (is_zero(D[pk_flag((TR == 0) != BACK)])) {
+    if (is_zero(D[pk_flag((TR == 0) != BACK, sd)])) {
         if (tid >= 64) return;
         // four lanes per unknown; the terms outside the triangle are left out, not multiplied by zero (an infinity in y
         // reaches the unknowns that depend on it, as in a substitution)
@@ -257,8 +259,8 @@ __device__ __forceinline__ void diag_solve(const T *D, int w, const T *y, PUT pu
 #pragma unroll
         for (int z = 0; z < 4; z++) {
             const int k = 8 * (q & 1) + 4 * (q >> 1) + z;         // (no bank conflicts in either order)
-            const T m = TR == 0 ? D[pk_e(o, k)] : opv<TR>(D[pk_e(k, o)]);
-            const bool in = BACK ? k >= o && k < w : k <= o;
+            const bool in = BACK ? k >= o && k < w : k <= o && o < w;
+            const T m = o >= sd || k >= sd ? VT<T>::zero() : TR == 0 ? D[pk_e(o, k, sd)] : opv<TR>(D[pk_e(k, o, sd)]);
 #pragma unroll
             for (int r = 0; r < RB; r++) a[r] = madd<T>(a[r], m, in ? y[k * RB + r] : VT<T>::zero());
         }
@@ -270,7 +272,7 @@ __device__ __forceinline__ void diag_solve(const T *D, int w, const T *y, PUT pu
         return;
     }
     if (tid >= 32 * sub_warps(RB)) return;
-    const T x = diag_sub<T, TR, BACK, UNIT, RB>(D, w, y);
+    const T x = diag_sub<T, TR, BACK, UNIT, RB>(D, sd, w, y);
     if (RB > 1 || tid < 16) put(tid & 15, RB == 1 ? 0 : 2 * (tid >> 5) + ((tid >> 4) & 1), x);
 }
 
@@ -306,7 +308,7 @@ __device__ __forceinline__ void chain_tri(const T *tr, T *ys, T *x, int np, int 
             named_bar(1, CH_THREADS);
         }
         if (threadIdx.x < diag_threads(RB))
-            diag_solve<T, TR, TR == 0, false, RB, false>(D, np - k0 < 16 ? np - k0 : 16, ys + k0 * RB,
+            diag_solve<T, TR, TR == 0, false, RB, false>(D, 16, np - k0 < 16 ? np - k0 : 16, ys + k0 * RB,
                                                          [&](int i, int r, T v) { x[(k0 + i) * RB + r] = v; });
         named_bar(1, CH_THREADS);
         if (TR == 0 && b > 0) {
@@ -707,7 +709,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__rest
             const T *D = ring + (done % CH_LSTAGES) * psz, *Lp = D + 256;      // Lp[c * rl + (row - k0 - w)]
             if (TR == 0) {
                 if (tid < diag_threads(RB))
-                    diag_solve<T, 0, false, true, RB, true>(D, w, v + k0 * RB, [&](int i, int r, T a) {
+                    diag_solve<T, 0, false, true, RB, true>(D, 16, w, v + k0 * RB, [&](int i, int r, T a) {
                         if (i < w) { v[(k0 + i) * RB + r] = a; if (r < rb) S2[F.f + k0 + i + r * n] = a; }
                     });
                 else if (loader) load_next();
@@ -760,7 +762,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_chain_l(const ChainFront *__rest
                 }
                 __syncthreads();
                 if (tid < diag_threads(RB))
-                    diag_solve<T, TR, true, true, RB, true>(D, w, v + k0 * RB, [&](int i, int r, T a) {
+                    diag_solve<T, TR, true, true, RB, true>(D, 16, w, v + k0 * RB, [&](int i, int r, T a) {
                         if (i < w) { v[(k0 + i) * RB + r] = a; if (r < rb) S2[F.f + k0 + i + r * n] = a; }
                     });
             }

@@ -115,10 +115,14 @@ static int upload_segments(int64_t n, const std::vector<int64_t> &Bp, DevPlan &D
 static const int64_t SV_MAXDIM = 768, SV_MAXNP = 64, SV_MAXBLK = 32768;
 // front fi's packed pieces (k_front_pack): their offsets from *size on, which moves past them, and the rows of its L pieces (all
 // of the front's where the one-launch chain sweeps read them)
-static void pack_layout(const FrontPlan &P, const DevPlan &D, int64_t fi, long long *u_pk, long long *l_pk, long long *l_rows, int64_t *size)
+static void pack_layout(const FrontPlan &P, const DevPlan &D, int64_t fi, long long *u_pk, long long *l_pk, long long *l_rows, long long *side,
+                        int64_t *size)
 {
     const Front &F = P.fronts[(size_t)fi];
-    const int64_t np = std::min(F.npiv, F.nrows), nb = (np + 15) / 16, R = D.ch_count > 0 && fi >= D.chain_begin ? F.nrows : np;
+    const bool chain = D.ch_count > 0 && fi >= D.chain_begin;
+    const int64_t np = std::min(F.npiv, F.nrows), nb = (np + 15) / 16, R = chain ? F.nrows : np;
+    *side = chain ? 16 : pk_side(np);
+    if (nb == 1 && *side < 16) { *u_pk = *size; *l_pk = *size + *side * *side; *l_rows = R; *size = *l_pk + *side * *side; return; }
     *u_pk = *size;
     *l_pk = *size + pk_u(nb);
     *l_rows = R;
@@ -138,8 +142,8 @@ static int upload_solve_levels(const FrontPlan &P, DevPlan &D, char *err, size_t
     D.sv_cols_maxnc.assign((size_t)nlev, 0); D.sv_cols_maxnp.assign((size_t)nlev, 0);
     for (int64_t fi = 0; fi < nf; fi++) {
         const Front &F = P.fronts[fi];
-        sv[(size_t)fi] = SvFront{F.f, F.npiv, F.nrows, F.nri, F.ncols, F.L_off, F.U_off, F.row_off, F.col_off, 0, 0, D.dblk, 0, 0, 0};
-        pack_layout(P, D, fi, &sv[(size_t)fi].u_pk, &sv[(size_t)fi].l_pk, &sv[(size_t)fi].l_rows, &D.pk_size);
+        sv[(size_t)fi] = SvFront{F.f, F.npiv, F.nrows, F.nri, F.ncols, F.L_off, F.U_off, F.row_off, F.col_off, 0, 0, D.dblk, 0, 0, 0, 0};
+        pack_layout(P, D, fi, &sv[(size_t)fi].u_pk, &sv[(size_t)fi].l_pk, &sv[(size_t)fi].l_rows, &sv[(size_t)fi].pk_s, &D.pk_size);
         for (int64_t b = 0; b < (std::min(F.npiv, F.nrows) + 15) / 16; b++) dfront.push_back((int)fi);
         D.dblk = (int64_t)dfront.size();
         const size_t L = (size_t)F.level;
@@ -372,9 +376,9 @@ int dev_upload_plan(const fplus_symbolic *S, const FrontPlan &P, DevPlan &D, cha
             if (one && uo_ok && chain_l_smem(mnr, 1, 16) <= 220 * 1024) {
                 D.ch_count = nf - c0; D.ch_maxnr = mnr; D.ch_u0 = P.fronts[c0].U_off; D.ch_nplast = P.fronts[nf - 1].npiv;
                 int64_t pks = 0;
-                long long up = 0, lp = 0, lr = 0;
+                long long up = 0, lp = 0, lr = 0, sd = 0;
                 for (int64_t j = 0; j < nf; j++) {
-                    pack_layout(P, D, j, &up, &lp, &lr, &pks);
+                    pack_layout(P, D, j, &up, &lp, &lr, &sd, &pks);
                     if (j >= c0) { cf[(size_t)(j - c0)].u_pk = up; cf[(size_t)(j - c0)].l_pk = lp; }
                 }
                 if ((rc = upload(cf, &D.ch_fronts, err, errlen))) return rc;

@@ -73,7 +73,7 @@ struct OutMap {
 struct SvFront {
     long long f, np, nr, nri, nc, L_off, U_off, row_off, col_off;
     long long nch, poff;           // the U sweep of a larger front: CB-column chunks, first partial sum (per right-hand side)
-    long long d_off, u_pk, l_pk, l_rows;   // its first 16-pivot block, its packed pieces (k_front_pack)
+    long long d_off, u_pk, l_pk, l_rows, pk_s;   // its first 16-pivot block, its packed pieces (k_front_pack)
 };
 
 // a front as the batched factorization kernels read it: its shape, arenas and row / column entries, its assembly entries

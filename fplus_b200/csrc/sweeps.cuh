@@ -7,7 +7,7 @@ namespace fpl {
 constexpr int SW_THREADS = 256;
 
 // A front's triangle applied to the vector x (x[k * RB + r], k up to np and zero from there to the next sixteen, shared
-// memory; overwritten), the result in xs (the same layout): xs = L11^-1 x (UPPER false) or U11^-1 x.  By 16-column blocks: the
+// memory; overwritten; sd: the side of the front's diagonal blocks, less than 16 only for a single one), the result in xs (the same layout): xs = L11^-1 x (UPPER false) or U11^-1 x.  By 16-column blocks: the
 // block's 16 unknowns (diag_solve), then the rows beyond it updated from the block's
 // columns; the packed pieces (at pk, see k_front_pack) stream through a ring of STG stages of psz elements by bulk copies
 // ahead of the chain.  The pipe (its barriers, initialised, and the pieces taken so far) serves several calls of a CTA of
@@ -17,7 +17,7 @@ constexpr int SW_THREADS = 256;
 struct TriPipe { unsigned long long *bars; int done; };
 __host__ __device__ constexpr int tri_pad(int np) { return (np + 15) & ~15; }
 template <typename T, bool UPPER, int RB, int STG>
-__device__ __forceinline__ bool tri16(const T *__restrict__ pk, int np, T *x, T *xs, T *ring, int psz, TriPipe &pipe)
+__device__ __forceinline__ bool tri16(const T *__restrict__ pk, int sd, int np, T *x, T *xs, T *ring, int psz, TriPipe &pipe)
 {
     const int tid = threadIdx.x, nbk = (np + 15) >> 4;
     int issued = 0;
@@ -25,7 +25,7 @@ __device__ __forceinline__ bool tri16(const T *__restrict__ pk, int np, T *x, T 
     auto load_next = [&]() {                           // one thread
         if (issued >= nbk) return;
         const int b = blk(issued), k0 = 16 * b, w = np - k0 < 16 ? np - k0 : 16, sl = (pipe.done + issued) % STG;
-        const unsigned bytes = (unsigned)((256 + 16 * (UPPER ? k0 : np - k0 - w)) * sizeof(T));
+        const unsigned bytes = (unsigned)((sd * sd + 16 * (UPPER ? k0 : np - k0 - w)) * sizeof(T));
         bulk_expect(pipe.bars + sl, bytes);
         bulk_load(ring + sl * psz, pk + (UPPER ? pk_u(b) : pk_l(b, np)), bytes, pipe.bars + sl);
         issued++;
@@ -39,7 +39,7 @@ __device__ __forceinline__ bool tri16(const T *__restrict__ pk, int np, T *x, T 
         const T *D = ring + (d % STG) * psz, *Lp = D + 256;
         if (tid == SW_THREADS - 1) load_next();
         if (tid < diag_threads(RB))
-            diag_solve<T, 0, UPPER, !UPPER, RB, false>(D, w, x + k0 * RB, [&](int i, int r, T v) { xs[(k0 + i) * RB + r] = v; });
+            diag_solve<T, 0, UPPER, !UPPER, RB, false>(D, sd, w, x + k0 * RB, [&](int i, int r, T v) { xs[(k0 + i) * RB + r] = v; });
         __syncthreads();
         // the rows beyond the block: two lanes per row, eight columns each (columns beyond the pivots are zero)
         const int ra = UPPER ? 0 : k0 + w, rl = UPPER ? k0 : np - k0 - w;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_fwdL(const SvFront *__restric
             if (k < np) x[k * RB + r] = val; else v[k - np + r * m] = val;
         }
         __syncthreads();
-        if (!tri16<T, false, RB, 2>(pk + F.l_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+        if (!tri16<T, false, RB, 2>(pk + F.l_pk, (int)F.pk_s, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
         for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; Y[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
         for (int t = tid; t < m; t += SW_THREADS) {
             T acc[RB];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_bwdU(const SvFront *__restric
             x[ii * RB + r] = sub(Y[F.f + ii + (int64_t)(r0 + r) * n], s);
         }
         __syncthreads();
-        if (!tri16<T, true, RB, 2>(pk + F.u_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+        if (!tri16<T, true, RB, 2>(pk + F.u_pk, (int)F.pk_s, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
         for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; X[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
         __syncthreads();
     }
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_L11(const SvFront *__restric
         x[k * RB + r] = k < np && r < rc ? VB[F.row_off + k + (int64_t)(r0 + r) * vstride] : VT<T>::zero();
     }
     __syncthreads();
-    if (!tri16<T, false, RB, STG>(pk + F.l_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+    if (!tri16<T, false, RB, STG>(pk + F.l_pk, (int)F.pk_s, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
     for (int e = tid; e < np * rc; e += SW_THREADS) {
         const int k = e % np, r = e / np;
         VB[F.row_off + k + (int64_t)(r0 + r) * vstride] = xs[k * RB + r];
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_swb_bwdU(const SvFront *__restri
         x[i * RB + rr] = v;
     }
     __syncthreads();
-    if (!tri16<T, true, RB, STG>(pk + F.u_pk, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
+    if (!tri16<T, true, RB, STG>(pk + F.u_pk, (int)F.pk_s, np, x, xs, ring, psz, pipe)) { if (tid == 0) set_status(st, ST_WAIT, F.f, 0, 0); return; }
     for (int e = tid; e < np * rc; e += SW_THREADS) { const int k = e % np, r = e / np; X[F.f + k + (int64_t)(r0 + r) * n] = xs[k * RB + r]; }
 }
 

@@ -211,3 +211,40 @@ def test_device_bytes_count_the_packed_triangles(gpu):
     entries = int((P["nrows"] * npiv + npiv * (nc - npiv)).sum())
     packed = 512 * int((npiv >= 16).sum())          # fronts of one block: its upper and its lower triangle
     assert N.info["device_bytes"] >= 8 * (entries + packed) + 2 * 8 * A.nnz
+
+
+def test_small_fronts_pack_small(gpu):
+    """Fronts of a few pivots (here mostly one) take a few packed entries each, not whole 16 x 16 blocks."""
+    n = 60000
+    rng = np.random.default_rng(0)
+    A = (sp.identity(n) * 4.0 + sp.coo_matrix((rng.standard_normal(n // 4), (rng.integers(0, n, n // 4), rng.integers(0, n, n // 4))),
+                                              shape=(n, n))).tocsc()
+    m = n, A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data
+    S = F.analyze(*m[:3])
+    N = S.factor(A.data)
+    assert np.bincount(S.plan()["col_front"]).mean() < 1.5
+    assert N.info["device_bytes"] < 24e6            # (over 180 MB with a block each)
+    for nrhs in (1, 9):
+        _check(m, S, N, nrhs, 0)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_one_block_fronts(gpu, cplx):
+    """Independent dense blocks of 1 to 20 pivots: every side of a packed block, in product and in substitution form."""
+    rng = np.random.default_rng(5)
+    blocks = []
+    for k in range(1, 21):
+        B = rng.standard_normal((k, k)) + (1j * rng.standard_normal((k, k)) if cplx else 0)
+        blocks.append(B)
+        if k > 2:
+            B = B.copy()
+            B[:, k - 2] = B[:, :k - 2] @ rng.uniform(-1, 1, k - 2) + 1e-6 * B[:, k - 2]
+            blocks.append(B)
+    A = sp.block_diag([sp.coo_matrix(B) for B in blocks], format="csc")
+    A.sort_indices()
+    m = A.shape[0], A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data.copy()
+    S = F.analyze(*m[:3])
+    N = S.factor(m[3])
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        for nrhs in (1, 2, 8, 9):
+            _check_from_x(m, N, nrhs, trans)
