@@ -169,16 +169,14 @@ enum : int {
     ST_SOLVE_ZERO = 5,     // a zero diagonal of U in a solve
     ST_BAD_VALUE = 6,      // a non-finite input value at idx
     ST_RANGE = 7,          // a captured factorization met values beyond 2^+-500 (the range guard needs the host path)
-    ST_WAIT = 8,           // a wait of a multi-CTA pivot search for the other CTAs' candidates ran out of time
+    ST_WAIT = 8,           // a wait for other CTAs of a launch, or for a bulk copy, ran out of time
 };
 struct DevStatus {
     int code;
     int pad;
     long long idx;
     double best, thr;
-    // Ruiz
-    unsigned long long res_bits;   // max |log| residual of the running iteration (bits of a non-negative double)
-    int done, iters;
+    int iters, pad2;               // Ruiz: the iterations that ran
     unsigned long long amax_bits, amin_bits;
     unsigned int ticket;           // CTAs of the running fused backward-sweep launch that have finished (0 between launches)
     unsigned int tc_err;           // a tensor-core Schur update whose wait ran out of time (bits, see schur_tc.hpp)

@@ -1422,7 +1422,8 @@ static int run_solve_block(const FrontPlan &P, const DevPlan &D, DevNum &N, T *x
                                                               nrhs), note_launch();
                 if (mnp > 0) {
                     // the L11 solves: at most 8 right-hand sides per CTA (the groups in parallel); by 16-column blocks while
-                    // shared memory holds two of them, else (more than 256 complex, 512 real pivots) by 64-row substitution
+                    // shared memory holds two of them, else (more than 282 complex or 576 real pivots with several
+                    // right-hand sides, 399 or 813 with one) by 64-row substitution
                     const int stg = tri_stages(mnp);
                     if (stg) {
                         auto kern = nrhs == 1 ? (stg == 3 ? k_swb_L11<T, 1, 3> : k_swb_L11<T, 1, 2>) : (stg == 3 ? k_swb_L11<T, 8, 3> : k_swb_L11<T, 8, 2>);

@@ -78,7 +78,7 @@ template <int STG> __device__ __forceinline__ TriPipe tri_pipe(unsigned long lon
 // shared memory of tri16 (x, xs and the ring), in elements
 static inline int64_t tri16_elems(int64_t np, int64_t rb, int stg) { return 2 * tri_pad((int)np) * rb + stg * (16 * np + 256); }
 
-// L sweep of a level's small fronts, a CTA each (the successor of k_sv_fwdL): the front's vector in its final row order, x =
+// L sweep of a level's small fronts, a CTA each: the front's vector in its final row order, x =
 // L11^-1 v (into Y in pivot order), then the contribution u = v[np:] - L21 x into VB, a thread per row with L's row read
 // once for all of the pass's right-hand sides
 template <typename T, int RB>
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(SW_THREADS) k_sw_fwdL(const SvFront *__restric
 }
 static inline int64_t sw_fwdL_elems(int64_t nr, int64_t np, int64_t rb) { return nr * rb + tri16_elems(np, rb, 2); }
 
-// U sweep of a level's small fronts, a CTA each (the successor of k_sv_bwdU): the CB columns' x gathered into shared memory,
+// U sweep of a level's small fronts, a CTA each: the CB columns' x gathered into shared memory,
 // the product with U12 split over column groups (each U12 entry read once for all of the pass's right-hand sides; the
 // groups' sums added in order), then x = U11^-1 (y - the product)
 template <typename T, int RB>

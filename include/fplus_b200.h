@@ -142,8 +142,8 @@ void fplus_b200_graph_free(fplus_b200_graph *graph);
 
 /* The front-shape autotuner (no counterpart in FPLUS): factors the given values once per candidate shape of the
  * multifrontal structure (at most 128, 256 or 512 pivot columns per front, the panel width of the large fronts' Schur
- * updates; for a pattern with a dense chain also 32 or 64 pivots per chain front), then the best shape with the blocked
- * pivot-block LU, each timed on the device twice (permutation, Ruiz and the fronts), in the given precision
+ * updates; for a pattern with a dense chain also 32 or 64 pivots per chain front), then the best shape with the
+ * shared-memory pivot-block LU (variant 1), each timed on the device twice (permutation, Ruiz and the fronts), in the given precision
  * (FPLUS_B200_PREC_*), and keeps the fastest in sym for every later factorization on it.  The pivots do not depend on the shape.  best_width, best_nb, best_ms may be NULL. */
 int fplus_b200_autotune(fplus_symbolic *sym, const int64_t *Ap, const int64_t *Ai, const void *Ax, int is_complex,
                         const fplus_options *opt, int precision, int64_t *best_width, int64_t *best_nb, int *best_lu,
@@ -151,10 +151,9 @@ int fplus_b200_autotune(fplus_symbolic *sym, const int64_t *Ap, const int64_t *A
 
 /* The front shape of every later factorization on sym, chosen by the caller instead of the autotuner: at most max_width
  * pivot columns per front (16 .. 4096), nb_chain pivots per dense-chain front (8 .. 64), and the pivot-block LU of the
- * small fronts (2: 8-column panels with the later
- * columns' updates on the FP64 tensor cores, the default; 1: the block in shared memory, one barrier per pivot step; 3:
- * blocked 8-column panels in FP64 lanes), plus 4 to pivot the pivot blocks too large for one CTA by one CTA per 32-column panel
- * instead of all SMs in one launch, plus 8 to factor every front on its own instead of the small fronts at the bottom of
+ * small fronts (2: 8-column panels with the later columns' updates on the FP64 tensor cores, the default; 1: the block in
+ * shared memory, one barrier per pivot step; 3: blocked 8-column panels in FP64 lanes), plus 4 to pivot the pivot blocks too
+ * large for one CTA by one CTA per 32-column panel instead of a cluster or all SMs in one launch, plus 8 to factor every front on its own instead of the small fronts at the bottom of
  * the tree level by level (variant 3 also turns that off), plus 16 to form the small fronts' U12 and contribution blocks
  * by 16-row forward-substitution steps instead of products with the inverted diagonal blocks, plus 32 to pass the
  * pipelined fronts' contribution blocks through the stack instead of writing them into the parent's working block.  The
