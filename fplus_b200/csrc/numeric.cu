@@ -978,11 +978,13 @@ static int run_fronts(const FrontPlan &P, const DevPlan &D, DevNum &N, double pi
             prof.end(s);
             if (D.bs_maxtiles[(size_t)lv] > 0) {
                 prof.begin(s, PROF_SCHUR, fm * D.bs_tail_flops[(size_t)lv], D.bs_tail_bytes[(size_t)lv] * (double)vs);
-                const dim3 tg((unsigned)std::min<int64_t>(D.bs_maxtiles[(size_t)lv], 148), cnt);
-                if (!(N.lu_variant & 16))
-                    k_bat_tail2<T, FT_TN><<<tg, FT_THREADS, fsm, s>>>(D.fc, bl, Wb, N.permall, La, Ua, CBA, N.st), note_launch();
-                else
-                    k_bat_tail<T, FT_TN><<<tg, FT_THREADS, fsm, s>>>(D.fc, bl, Wb, N.permall, La, Ua, CBA, N.st), note_launch();
+                for (unsigned c0 = 0; c0 < cnt; c0 += 65535) {            // (the most CTAs in a grid's second dimension)
+                    const dim3 tg((unsigned)std::min<int64_t>(D.bs_maxtiles[(size_t)lv], 148), std::min(cnt - c0, 65535u));
+                    if (!(N.lu_variant & 16))
+                        k_bat_tail2<T, FT_TN><<<tg, FT_THREADS, fsm, s>>>(D.fc, bl + c0, Wb, N.permall, La, Ua, CBA, N.st), note_launch();
+                    else
+                        k_bat_tail<T, FT_TN><<<tg, FT_THREADS, fsm, s>>>(D.fc, bl + c0, Wb, N.permall, La, Ua, CBA, N.st), note_launch();
+                }
                 prof.end(s);
             }
         }

@@ -2,6 +2,7 @@
 worker streams and captured as one CUDA graph, against the same calls made one by one."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import fplus_b200 as F
 from fplus_b200 import workloads as W
@@ -72,3 +73,18 @@ def test_worker_batch_matches_one_by_one(gpu):
     assert F.batch_span_ms(Ns) > 0.0
     for S, m, b, X in zip(syms, mats, rhs, Xs):
         assert np.array_equal(X, S.factor(m[3]).solve(b))
+
+
+def test_level_of_many_fronts(gpu):
+    """More fronts in one level of the tree than a grid's second dimension takes (65,535): mostly one-pivot fronts."""
+    n = 150000
+    rng = np.random.default_rng(0)
+    A = (sp.identity(n) * 4.0 + sp.coo_matrix((rng.standard_normal(n // 4), (rng.integers(0, n, n // 4), rng.integers(0, n, n // 4))),
+                                              shape=(n, n))).tocsc()
+    m = n, A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data
+    S = F.analyze(*m[:3])
+    assert (S.plan()["parent"] < 0).sum() > 65535
+    b = A @ rng.uniform(-1, 1, n)
+    for variant in (2, 18):
+        S.set_front_shape(256, 64, variant)
+        assert O.backward_error(*m, S.factor(A.data).solve(b), b) <= 1e-14
