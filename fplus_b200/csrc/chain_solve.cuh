@@ -42,11 +42,14 @@ struct ChainFront {
 // The diagonal block is kept as its inverse D (identity beyond the pivots) or as the triangle itself (U: with the reciprocals
 // of the pivots on its diagonal; one beyond the pivots); which, says the far corner of the other triangle (pk_flag: zero for
 // the inverse).  A tree front of at most 8 pivots has a block of 2, 4 or 8 rows and columns (side s) instead of 16: with 256
-// elements for every one-pivot front a diagonal matrix's packed triangles were 512 times its factors.  x = D y leaves a residual of at most about u |U| |D| |U| |x| where substitution leaves u |U| |x|, so the inverse
-// stands only where || |U| |D| ||_1 <= PACK_GROWTH.  Backward errors of x = D y, blocks with a column within 1 to 1e-8.5 of the
-// ones before it: at most 1e-17 times that norm (4e-15 at 1,000, 3e-9 at 3e8; substitution 6e-17 throughout).  The norm (of
-// |re| + |im|) is 2 to 9 on the stencils' and the random matrices' fronts; on the pencils' chains 45 to 50 in the middle (U) and
-// at most 81 (L), about 4 blocks of 100 above 128; on a narrow complex band's 124 in the middle.
+// elements for every one-pivot front a diagonal matrix's packed triangles were 512 times its factors.
+// x = D y leaves a residual of up to about u |U| |D| |U| |x| where substitution leaves u |U| |x|.  So the inverse stands only where
+// the 1-norms of R^-1 |U| |D| R and of C^-1 |U|^T |D|^T C (the transposed sweeps) are at most PACK_GROWTH; R and C hold the
+// block's row and column sums, so that a scaling of the rows or columns changes nothing.  Measured over blocks with a column
+// within 1 to 1e-8.5 of the ones before it, rows scaled over up to 16 decades: the largest row's |r| / (|U| |x| + |y|) is at
+// most 1.4e-16 times the norm for x = D y (where D stands: 7e-15, 1.5e-16 in the middle), 2.3e-16 for substitution.  The norms
+// (of |re| + |im|) are at most 7 on the stencils' and the random matrices' fronts; on the pencils' chains about 22 in the
+// middle, at most 33 (L), 1 block of 100 above 128 (U); on narrow complex bands' 33 to 51 in the middle, 1 to 25 of 100 above.
 __host__ __device__ constexpr int64_t pk_u(int64_t b) { return 256 * b + 128 * b * (b - 1); }
 __host__ __device__ constexpr int64_t pk_l(int64_t b, int64_t R) { return 256 * b + 16 * b * R - 128 * b * (b + 1); }
 __host__ __device__ constexpr int pk_e(int i, int k, int s = 16) { return s * k + ((i + k) & (s - 1)); }
@@ -89,12 +92,28 @@ __global__ void __launch_bounds__(128) k_front_pack(const SvFront *__restrict__ 
                 x[i] = i < w ? (is_zero(d) ? VT<T>::zero() : mul(s, recip(d))) : s;
             }
         }
-        // the norm: the column sums of the block's moduli times the moduli of the inverse's column, the largest column
-        double cs = lower || c >= w ? 1.0 : 0.0, g = 0.0;
-        for (int i = lower ? c + 1 : 0; i < (lower ? 16 : c + 1); i++) cs += abs1(at(i, c));
+        // the two norms (of the block and of its transpose): lane c has row c's sum of moduli and column c's, then the sums over
+        // the other direction's divided by them, then one entry of each norm; an inverse, a sum or a quotient out of range
+        // makes it infinite or NaN
+        auto mod = [&](int i, int k) -> double { return i == k && (lower || i >= w) ? 1.0 : (lower ? i >= k : i <= k) ? abs1(at(i, k)) : 0.0; };
+        double rs = 0.0, cs = 0.0, rq = 0.0, cq = 0.0, g = 0.0, gt = 0.0;
+        for (int k = 0; k < 16; k++) { rs += mod(c, k); cs += mod(k, c); }
+        const double ri = 1.0 / rs, ci = 1.0 / cs;
+        for (int k = 0; k < 16; k++) {
+            cq += mod(k, c) * __shfl_sync(0xffffffffu, ri, k, 16);
+            rq += mod(c, k) * __shfl_sync(0xffffffffu, ci, k, 16);
+        }
 #pragma unroll
-        for (int i = 0; i < 16; i++) g += __shfl_sync(0xffffffffu, cs, i, 16) * abs1(x[i]);
-        const unsigned good = __ballot_sync(0xffffffffu, g <= PACK_GROWTH);     // (not where the inverse overflows: NaN, infinity)
+        for (int k = 0; k < 16; k++) {
+            const double m = abs1(x[k]);
+            g += __shfl_sync(0xffffffffu, cq, k, 16) * m;
+            double t = m * rq;
+            for (int h = 8; h > 0; h >>= 1) t += __shfl_xor_sync(0xffffffffu, t, h);
+            if (k == c) gt = t;
+        }
+        g *= rs;
+        gt *= cs;
+        const unsigned good = __ballot_sync(0xffffffffu, g <= PACK_GROWTH && gt <= PACK_GROWTH);
         const bool inv = (lower ? good >> 16 : good & 0xffffu) == 0xffffu;
         T *o = lower ? dl : du;
 #pragma unroll

@@ -176,6 +176,35 @@ def test_ill_conditioned_diagonal_blocks(gpu, cplx, where, kind, n):
             _check_from_x(m, N, nrhs, trans)
 
 
+def _row_error(m, x, b, trans):
+    A = sp.csc_matrix((m[3], m[2], m[1]), shape=(m[0], m[0]))
+    A = {0: A, 1: A.T, 2: A.conj().T}[trans]
+    return float((abs(A @ x - b) / (abs(A) @ abs(x) + abs(b))).max())
+
+
+@pytest.mark.parametrize("where", ["tree", "chain"])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_graded_rows(gpu, cplx, where):
+    """Every row's residual is small beside that row (or column, transposed) of an upper triangular matrix: 16 x 16 blocks of
+    0.1 and -1 whose rows grow a hundredfold each (a large inverse that norms of the unscaled block do not show)."""
+    n = 112
+    m = _hard("upper", n, cplx, 1)
+    A = m[3].reshape(n, n).T * 100.0 ** (np.arange(n) % 16)[:, None]
+    eye = np.arange(n, dtype=np.int64)
+    for trans in ((0, 1, 2) if cplx else (0, 1)):
+        # (transposed: the columns grow, towards the first)
+        B = A if trans == 0 else m[3].reshape(n, n).T * 100.0 ** (15 - np.arange(n) % 16)[None, :]
+        mm = (*m[:3], np.ascontiguousarray(B.T).ravel())
+        S = F.Symbolic.from_orders(*mm[:3], eye, eye) if where == "chain" else F.analyze(*mm[:3], pin_dense=0)
+        N = S.factor(mm[3], F.default_options(equilibrate=0, pivot_rel=0.0, pin_dense=0))
+        assert np.array_equal(N.p, eye)
+        for nrhs in (1, 9):
+            x = np.random.default_rng(nrhs).uniform(-1, 1, (n, nrhs))
+            C = {0: B, 1: B.T, 2: B.conj().T}[trans]
+            y = N.solve(C @ x, trans)
+            assert max(_row_error(mm, y[:, r], (C @ x)[:, r], trans) for r in range(nrhs)) <= 1e-14
+
+
 @pytest.mark.parametrize("delta", [1e-4, 1e-7])
 @pytest.mark.parametrize("nb", [32, 64])
 @pytest.mark.parametrize("cplx", [False, True])
