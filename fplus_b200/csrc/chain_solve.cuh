@@ -234,13 +234,13 @@ __device__ __forceinline__ void quad_mv(T (&acc)[RB], const T *Mp, int ld, int o
 }
 
 // x = M^-1 y for a packed 16 x 16 diagonal block D of w <= 16 unknowns: M = L (unit lower) or U (TR 0), or its transpose (TR 1, 2
-// with conj); BACK: M is upper triangular; UNIT: it has a unit diagonal; sd: the block's side (w <= sd).  y: [k * RB + r], finite or not, zero from w on or not
-// part of the block.  By the threads tid < diag_threads(RB); put(o, r, x) takes unknown o < 16 of right-hand side r, zero from
+// with conj); BACK: M is upper triangular; UNIT: it has a unit diagonal; sd: the block's side (w <= sd).  y: [k * RB + r], finite
+// or not, from w on zero or not part of the block.  By the threads tid < diag_threads(RB); put(o, r, x) takes unknown o < 16 of right-hand side r, zero from
 // w on (INPLACE: after every thread has read y; named barrier 2).
 //
-// What bounds it (B200, one right-hand side, from y in shared memory to x there, two barriers included): the product 263
-// cycles real, 461 complex; the substitution, a lane per unknown and one exchange per step, 970 (unit) and 1,480 real, 1,630
-// and 1,890 complex (a dependent FP64 operation takes about 25 cycles, a shuffle 27).  Four unknowns at a time, solved by every
+// What bounds it (B200, one right-hand side, from y in shared memory to x there, two barriers included): the product 373
+// cycles real, 481 complex (263 and 461 without the flag and the terms left out; 1,238 and 1,066 with 8 and 4 right-hand
+// sides); the substitution, a lane per unknown and one exchange per step, 970 (unit) and 1,480 real, 1,630 and 1,890 complex (a dependent FP64 operation takes about 25 cycles, a shuffle 27).  Four unknowns at a time, solved by every
 // lane for itself, took 1,180 to 1,200 real and 1,780 to 1,890 complex; the whole block in one lane 960 to 3,080.
 __host__ __device__ constexpr int sub_warps(int rb) { return (rb + 1) / 2; }
 __host__ __device__ constexpr int diag_threads(int rb) { return 32 * sub_warps(rb) > 64 ? 32 * sub_warps(rb) : 64; }
